@@ -216,6 +216,8 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
     e->dims.byW = kH / 2;
     e->dims.bxW = kW / 2;
     e->dims.col_warps = cw;
+    e->dims.col_auto = col_warps == 0;
+    e->dims.wpitch = (dataW + 3) & ~3;
     e->dims.radix_step = kRadixDft;
     e->kH = kH;
     e->kW = kW;
@@ -235,7 +237,7 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
 
     const size_t plane = (size_t)dataH * dataW;
     bool ok = FMVD_CHECK(cudaMalloc(&e->spec, sizeof(float2) * e->spec_elems * 2 * nViews)) &&
-              FMVD_CHECK(cudaMalloc(&e->weights, sizeof(float) * plane * nViews)) &&
+              FMVD_CHECK(cudaMalloc(&e->weights, sizeof(float) * (size_t)dataH * e->dims.wpitch * nViews)) &&
               FMVD_CHECK(cudaMalloc(&e->C, sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
               FMVD_CHECK(cudaMalloc(&e->est, sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
               FMVD_CHECK(cudaMalloc(&e->twH, sizeof(float2) * H)) && FMVD_CHECK(cudaMalloc(&e->twW, sizeof(float2) * W)) &&
@@ -280,7 +282,7 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
                 ok = FMVD_CHECK(cudaMemcpy(d_k, src, sizeof(float) * kH * kW, cudaMemcpyHostToDevice));
                 if (ok) {
                     rl_kernel_spectrum(d_k, kH, kW, H, W, e->twH, e->twW, work,
-                                       e->spec + e->spec_elems * (2 * v + which), e->dims.col_warps, 0);
+                                       e->spec + e->spec_elems * (2 * v + which), 0);
                     ok = FMVD_CHECK(cudaGetLastError()) && FMVD_CHECK(cudaDeviceSynchronize());
                 }
             }
@@ -296,7 +298,7 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
         for (int v = 0; v < nViews && ok; v++)
             ok = FMVD_CHECK(cudaMemcpy(raw + plane * v, h_Weights[v], sizeof(float) * plane, cudaMemcpyHostToDevice));
         if (ok) {
-            rl_normalize_weights(raw, e->weights, nViews, plane, 0);
+            rl_normalize_weights(e->dims, raw, e->weights, 0);
             ok = FMVD_CHECK(cudaGetLastError()) && FMVD_CHECK(cudaDeviceSynchronize());
         }
         cudaFree(raw);

@@ -30,7 +30,7 @@ struct Engine {
     int device;
     size_t spec_elems;      // complex values per kernel spectrum (launch layout)
     float2 *spec;           // V x 2 spectra: [v][0] kernel 1, [v][1] kernel 2
-    float *weights;         // V x dataH x dataW normalised weights
+    float *weights;         // V x dataH x dims.wpitch normalised weights
     float2 *C;              // pairs_cap x H x W
     float2 *est;            // pairs_cap x H x W
     float2 *twH, *twW;      // exp(-2 pi i n / N), line engine (lengths above 1024)

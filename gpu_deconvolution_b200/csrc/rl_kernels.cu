@@ -40,10 +40,7 @@ static unsigned long long g_launches = 0;
 unsigned long long rl_launch_count() { return g_launches; }
 void rl_count_launch(unsigned long long n) { g_launches += n; }
 
-// Work planes are row-major (natural order): element (y, x) of pair p at
-// C[(p * H + y) * W + x].  Column blocks read runs of 4 to 8 complex values
-// (32 to 64 bytes, whole L2 sectors) per row.
-__host__ __device__ __forceinline__ size_t tile_index(int y, int x, int W) { return (size_t)y * W + x; }
+// Work planes are row-major: element (y, x) of pair p at C[(p * H + y) * W + x].
 
 __device__ __forceinline__ int clamp_src(int i, int n, int border)
 {
@@ -102,18 +99,9 @@ struct RowArgs {
     int view;
     int last;
     int bulk_data;      // data rows may be fetched with 16-byte bulk copies
-    int bulk_weights;   // weight rows may be fetched with 16-byte bulk copies
     int group_floats;   // warp engine: shared floats per group (transpose + prefetch)
     const float2 *twN;  // lines above 1024: exp(-2 pi i n / W), n < W
 };
-
-// Sample loads and estimate traffic are streamed (evict-first in L2) so that
-// the batch's complex work planes stay resident in L2 between passes.
-__device__ __forceinline__ float load_sample(const void *base, size_t idx, int bits)
-{
-    return bits == 16 ? (float)__ldcs(reinterpret_cast<const unsigned short *>(base) + idx)
-                      : (float)__ldcs(reinterpret_cast<const unsigned char *>(base) + idx);
-}
 
 // Float to sample as the reference's unpad kernel: clip at the maximum,
 // then convert with truncation (saturating at 0 for negatives).
@@ -135,23 +123,26 @@ __device__ __forceinline__ void store_sample(void *base, size_t idx, float v, in
 //           reference's in-place quirk)
 //   UPDATE: correction r -> e + w (e r - e) (multiply32_kernel); after the
 //           last view of the last iteration also the output samples
-// BITS: the sample width when fixed at compile time (8 or 16), else 0.  With
-// it fixed, operand rows are read through generic pointers that may point to
-// shared or global memory, so the element-wise step has no per-element
-// branches.  NOOUT: an update pass known at compile time not to be the last
-// one, so the output-sample code is left out.  SMEM (with BITS fixed): the
-// operand rows are in shared memory at the s_* addresses (the data rows in
-// the divide pass; the weight row in the update pass, and the estimate row
-// too when EST_S).
+// BITS: the sample width (8 or 16; 0 in the INIT pass, which has no samples),
+// so the element-wise step has no per-element branches.  NOOUT: an update pass
+// known at compile time not to be the last one, so the output-sample code is
+// left out.  SMEM: the operand row is in shared memory at the s_* addresses
+// (the data rows in the divide pass, where their alignment allows the bulk
+// copy; the weight row in the update pass, always, and the estimate row too
+// when EST_S).  Weight rows lie a multiple of 16 bytes apart so that the bulk
+// copy takes any plane width: with widths that are not a multiple of four the
+// rows used to be read element by element through generic pointers, 22.7 us
+// for an update of 8 pairs of 512 x 512 against 14.6.  (Rows padded to W,
+// which save the border arithmetic, cost more than they give: 4.2 % of a
+// 1024-point step, since the larger shared memory leaves less L1 for the
+// twiddle tables.)  Estimate traffic is streamed (evict-first in L2) so that
+// the batch's complex work planes stay resident between passes.
 template <int MODE, int BITS = 0, bool NOOUT = false, bool SMEM = false, bool EST_S = SMEM>
 struct RowWork {
     const RlDims &d;
     float2 *est;             // row y of the pair's estimate (global)
-    const float2 *est_s;     // the same row prefetched into shared memory, or null
     const void *src0, *src1; // data rows (clamped) of planes 2p and 2p+1, view a.view
-    bool src_s;              // data rows are in shared memory
     const float *wrow;       // weight row (clamped)
-    bool w_s;                // weight row is in shared memory
     void *out0, *out1;       // output rows, or null
     bool has1;
     float init0, init1;
@@ -163,7 +154,6 @@ struct RowWork {
         const int W = d.W;
         has1 = 2 * p + 1 < a.b.nplanes;
         est = a.b.est + ((size_t)p * d.H + y) * W;
-        est_s = nullptr;
         init0 = a.b.init_value;
         init1 = has1 ? a.b.init_value : 0.f;
         initr0 = initr1 = nullptr;
@@ -173,7 +163,6 @@ struct RowWork {
         }
         const size_t es = d.bits == 16 ? 2 : 1;
         src0 = src1 = nullptr;
-        src_s = w_s = false;
         wrow = nullptr;
         out0 = out1 = nullptr;
         if (MODE == ROW_DIVIDE) {
@@ -182,7 +171,7 @@ struct RowWork {
             src1 = has1 ? (const char *)a.b.data + (base + (size_t)(2 * p + 1) * a.b.plane_stride) * es : src0;
         }
         if (MODE == ROW_UPDATE) {
-            wrow = a.b.weights + (size_t)a.view * d.dataH * d.dataW + (size_t)clamp_src(y, d.dataH, d.byW) * d.dataW;
+            wrow = a.b.weights + ((size_t)a.view * d.dataH + clamp_src(y, d.dataH, d.byW)) * d.wpitch;
             if (a.last && y < d.dataH) {
                 out0 = (char *)a.b.out + ((size_t)(2 * p) * a.b.plane_stride + (size_t)y * d.dataW) * es;
                 if (has1)
@@ -195,12 +184,8 @@ struct RowWork {
     {
         if constexpr (BITS == 16)
             return (float)reinterpret_cast<const unsigned short *>(row)[sx];
-        else if constexpr (BITS == 8)
+        else
             return (float)reinterpret_cast<const unsigned char *>(row)[sx];
-        if (src_s)
-            return d.bits == 16 ? (float)reinterpret_cast<const unsigned short *>(row)[sx]
-                                : (float)reinterpret_cast<const unsigned char *>(row)[sx];
-        return load_sample(row, sx, d.bits);
     }
 
     __device__ __forceinline__ void apply(int x, float2 &v) const
@@ -227,31 +212,22 @@ struct RowWork {
             q.y = q.y > 1.f ? __fdividef(a1, q.y) : q.y;
             v = q;
         } else {
-            const int sx = clamp_src(x, d.dataW, d.bxW);
-            float w;
+            static_assert(MODE != ROW_UPDATE || SMEM, "the update pass reads its weight row from shared memory");
+            const float w = lds_f32(s_w + 4u * clamp_src(x, d.dataW, d.bxW));
             float2 c;
-            if constexpr (SMEM) {
-                w = lds_f32(s_w + 4u * sx);
-                if constexpr (EST_S)
-                    c = lds_f32x2(s_est + 8u * x);
-                else
-                    c = est[x];
-            } else if constexpr (BITS != 0) {
-                w = wrow[sx];
-                c = (est_s ? est_s : est)[x];
-            } else {
-                w = w_s ? wrow[sx] : __ldg(wrow + sx);
-                c = est_s ? est_s[x] : __ldcs(est + x);
-            }
+            if constexpr (EST_S)
+                c = lds_f32x2(s_est + 8u * x);
+            else
+                c = est[x];
             const float2 r = v;
             c.x += w * (c.x * r.x - c.x);
             c.y += w * (c.y * r.y - c.y);
             __stcs(est + x, c);
             v = c;
             if (!NOOUT && out0 && x < d.dataW) {
-                store_sample(out0, x, c.x, BITS ? BITS : d.bits);
+                store_sample(out0, x, c.x, BITS);
                 if (out1)
-                    store_sample(out1, x, c.y, BITS ? BITS : d.bits);
+                    store_sample(out1, x, c.y, BITS);
             }
         }
     }
@@ -272,6 +248,7 @@ struct RowWork {
 #define FMVD_COL_MAX_WARPS 8
 #endif
 constexpr int kRowWarps = 4;
+constexpr int kSms = 148;  // multiprocessors of a B200
 
 template <int W, int MODE, int BITS, bool NOOUT, bool SMEM>
 __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_w(const RowArgs a)
@@ -301,8 +278,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
     // lands in the transpose buffer itself, issued once the inverse
     // transform has read its transpose back, so it takes no shared memory
     // of its own.
-    // SMEM is set exactly when the launch allows the bulk copies (weights in
-    // the update pass, data in the divide pass)
+    // SMEM is set in the update pass, and in the divide pass exactly when the
+    // launch allows the bulk copies of the data rows
     constexpr bool prefetch = SMEM && MODE != ROW_INIT;
     uint64_t *bar = &bars[gi];
     uint64_t *ebar = &ebars[MODE == ROW_UPDATE ? gi : 0];
@@ -318,7 +295,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
     }
     if (prefetch && MODE == ROW_UPDATE && t == 0) {
         // the weight row is a plan constant: requested before the wait
-        const uint32_t wb = a.d.dataW * sizeof(float);
+        const uint32_t wb = a.d.wpitch * sizeof(float);
         mbar_arrive_expect_tx(bar, wb);
         bulk_load(pf, work.wrow, wb, bar);
     }
@@ -372,12 +349,11 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
         for (int m = 0; m < E; m++)
             v[m].y = -v[m].y;
     if (MODE == ROW_UPDATE) {
-        const bool ok_w = !prefetch || mbar_wait(bar, 0);
+        const bool ok_w = mbar_wait(bar, 0);
         const bool ok_e = mbar_wait(ebar, 0);
         if (!ok_w || !ok_e) {
             // a copy did not land in time: flag it (the host reports the
-            // batch as failed), wait once more so no copy is left in flight,
-            // and continue from global memory where the code allows it
+            // batch as failed) and wait once more so no copy is left in flight
             if (t == 0)
                 atomicExch(a.b.status, 1);
             if (!ok_w)
@@ -385,16 +361,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
             if (!ok_e)
                 mbar_wait(ebar, 0);
         }
-        if constexpr (SMEM) {
-            work.s_est = smem_u32addr(tbuf);
-            work.s_w = smem_u32addr(pf);
-        } else if (ok_w && ok_e) {
-            work.est_s = tbuf;
-            if (prefetch) {
-                work.wrow = reinterpret_cast<const float *>(pf);
-                work.w_s = true;
-            }
-        }
+        work.s_est = smem_u32addr(tbuf);
+        work.s_w = smem_u32addr(pf);
     } else if (prefetch) {
         if (!mbar_wait(bar, 0)) {
             // the copy did not land in time: flag it (the host reports the
@@ -456,47 +424,16 @@ __global__ void split_estimate_kernel(const float2 *__restrict__ est, int nplane
     }
 }
 
-// Column tile of the warp engine in shared memory: element (y, c) of the
-// block's FC columns.  With 32-lane groups the tile is dense and XOR-swizzled,
-// (y, c) at y * FC + (c ^ ((y >> SH) & (FC - 1))), SH = log2(32 / FC): the
-// coalesced row-wise fill, the per-column reads and the transposes of all
-// columns then each touch 32 distinct banks.  Smaller groups use a padded
-// row stride of FC + 1.
-template <int T, int FC>
-struct ColTile {
-    static constexpr bool swizzled = (T == 32) && FC > 1;
-    static constexpr int ld = swizzled ? FC : FC + 1;
-    static constexpr int sh = FC >= 32 ? 0 : (FC == 16 ? 1 : FC == 8 ? 2 : FC == 4 ? 3 : 4);
-    static __device__ __forceinline__ int at(int y, int c)
-    {
-        if constexpr (swizzled)
-            return y * FC + (c ^ ((y >> sh) & (FC - 1)));
-        else
-            return y * ld + c;
-    }
-    struct ColumnAddr {
-        int c;
-        __device__ __forceinline__ int operator()(int p) const { return at(p, c); }
-    };
-};
-
-// Interleaved (float2) column tile for 32-lane groups and 8 columns: element
-// (y, c) at y * 8 + (c ^ ((y >> 1) & 7)).  Sixteen consecutive rows of one
-// column then fall in sixteen distinct 8-byte slots of a 128-byte window, so
-// the per-column reads and both transpose phases (positions XOR-swizzled by
-// tpos) are free of bank conflicts with 64-bit accesses.
-struct ColTile2 {
-    static __device__ __forceinline__ int at(int y, int c) { return y * 8 + (c ^ ((y >> 1) & 7)); }
-    struct ColumnAddr {
-        int c;
-        __device__ __forceinline__ int operator()(int p) const { return at(p, c); }
-    };
-};
-
 // float2 shared-memory access by 32-bit shared-window address.
 __device__ __forceinline__ void sts2(uint32_t addr, float2 v)
 {
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ float4 lds4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ float2 lds2(uint32_t addr)
 {
@@ -505,145 +442,147 @@ __device__ __forceinline__ float2 lds2(uint32_t addr)
     return v;
 }
 
-// Byte addresses in a ColTile2 tile that starts on a 2048-byte boundary.
-// Slot (y, c) sits at byte 64 y + 8 (c ^ ((y >> 1) & 7)); for y = 32 a + u,
-// u < 32, that is 2048 a + Q_c(u) with Q_c(u) = 64 u + 8 (c ^ ((u >> 1) & 7)).
-// Q_c is XOR-linear: Q_c(t ^ k) = Q_c(t) ^ R(k), R(k) = 64 k + 8 ((k >> 1) & 7),
-// so every transpose address of the 1024-point column transform is a lane
-// constant XOR a compile-time constant (one logic instruction) plus an
-// immediate offset.
-__host__ __device__ constexpr uint32_t coltile_r(int k) { return 64u * k + 8u * ((k >> 1) & 7); }
+// Column tile of the warp engine (lengths up to 1024): FC columns as
+// interleaved float2, row y at byte 8 FC y, element (y, c) in 8-byte slot
+// c ^ f(y) of its row.  The engine moves 8-byte elements, sixteen lanes (one
+// 128-byte wavefront) at a time, and f spreads every access of a transform
+// over the sixteen slots of that wavefront:
+//   T = 32: sixteen lanes hold sixteen consecutive rows of one column, so f
+//     steps by one slot per 128 bytes of rows;
+//   T < 32: sixteen lanes hold eight (T = 4: four) rows of two (four)
+//     neighbouring columns, so f steps by two (four) slots and a column pair
+//     stays one aligned 16-byte unit: the tile is filled and written back 16
+//     bytes at a time.
+// With T = 16 the two lines of a warp are interleaved lane by lane (line =
+// lane & 1) to get eight rows of two columns in a half-warp.
+// f uses the low bits of y only, so that for u, k < T it is linear in XOR:
+// with the tile on a T * 8 FC byte boundary, the byte address of row
+// T a + (u ^ k) is 8 FC T a + (Q(u) ^ R(k)), Q(u) = 8 FC u + 8 (c ^ f(u)),
+// R(k) = 8 FC k + 8 f(k): one logic instruction on a lane constant and an
+// immediate offset per transpose access.
+template <int H, int FC>
+struct ColTile {
+    static constexpr int T = warp_fft_lanes(H);
+    static constexpr int RB = 8 * FC;                     // bytes per row
+    static constexpr int rows = T == 32 ? 32 : T < 8 ? 4 : 8;  // rows of a column that f tells apart
+    static constexpr int step = T == 32 ? 1 : 16 / rows;
+    static constexpr int sh = FC >= 16 ? 0 : FC == 8 ? 1 : FC == 4 ? 2 : 3;
+    static constexpr bool pairs = step > 1;               // column pairs stay adjacent
+    static constexpr uint32_t align = T * RB;
+    static constexpr size_t bytes = (size_t)H * RB + align;
+    static __host__ __device__ constexpr uint32_t f(int y) { return (((y & (rows - 1)) >> sh) * step) & (FC - 1); }
+    static __host__ __device__ constexpr uint32_t R(int k) { return (uint32_t)RB * k + 8u * f(k); }
+    // line (column of the warp) and lane inside the line
+    static __device__ __forceinline__ int line(int lane) { return T == 16 ? lane & 1 : lane / T; }
+    static __device__ __forceinline__ int pos(int lane) { return T == 16 ? lane >> 1 : lane % T; }
+};
 
-// 1024-point transform of one tile column (the WarpFft<1024> four-step with
-// T = E = 32): wbase = tile | Q_c(t) (transpose writes, element k1 at row
-// 32 k1 + (t ^ k1)), rbase = (tile + 2048 t) | Q_c(t) (reads of row-block t).
-template <int DIR>
-__device__ __forceinline__ void col_fft_1024(float2 *v, const float2 *__restrict__ tw, uint32_t wbase,
-                                             uint32_t rbase, int t)
+// H-point transform of one tile column (the WarpFft<H> four-step): wbase =
+// tile | Q(t) (transpose writes, element k1 at row T k1 + (t ^ k1 mod T)),
+// rbase = (tile + 8 FC T t) | Q(t) (reads of row-block t).
+template <int H, int FC, int DIR>
+__device__ __forceinline__ void col_fft(float2 *v, const float2 *__restrict__ tw, uint32_t wbase, uint32_t rbase, int t)
 {
-    Dft<32, DIR>::run(v);
-    WarpFft<1024>::twiddle<DIR>(v, tw, t);
+    using WF = WarpFft<H>;
+    using TL = ColTile<H, FC>;
+    constexpr int T = WF::T, E = WF::E, S = WF::S;
+    Dft<E, DIR>::run(v);
+    WF::template twiddle<DIR>(v, tw, t);
 #pragma unroll
-    for (int k1 = 0; k1 < 32; k1++)
-        sts2((wbase ^ coltile_r(k1)) + 2048u * k1, v[k1]);
+    for (int k1 = 0; k1 < E; k1++)
+        sts2((wbase ^ TL::R(k1 & (T - 1))) + (uint32_t)(T * TL::RB) * k1, v[k1]);
     __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 32; j++)
-        v[j] = lds2(rbase ^ coltile_r(j));
+    for (int s = 0; s < S; s++)
+#pragma unroll
+        for (int j = 0; j < T; j++)
+            v[s * T + j] = lds2((rbase ^ TL::R(j)) + (uint32_t)(T * T * TL::RB) * s);
     __syncwarp();
-    Dft<32, DIR>::run(v);
+#pragma unroll
+    for (int s = 0; s < S; s++)
+        Dft<T, DIR>::run(v + s * T);
+    WF::reorder(v);
 }
 
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
 // Column pass for H <= 1024: CW warps per block, G = 32 / T columns per
-// warp, FC = CW * G columns per block.  The FC-column tile is loaded into
-// shared memory with coalesced accesses, each group transforms its column in
-// registers using its own column of the tile as transpose buffer, and the tile
-// is written back.  Spectrum in launch layout: block bx, register m, thread
-// tid at spec[(bx * E + m) * (CW * 32) + tid].
+// warp, FC = CW * G columns per block.  The FC-column tile is filled by
+// cp.async (whole rows of the tile, 16 to 128 bytes, coalesced), each group
+// transforms its column in registers using its own column of the tile as
+// transpose buffer, and the tile is written back.  Spectrum in launch layout:
+// warp w of the plane (columns G w .. G w + G - 1), register m, lane l at
+// spec[(w * E + m) * 32 + l], whatever the block's width.
+// Bound by instruction issue (as the row passes): with the interleaved
+// XOR-swizzled tile a 512 x 512 launch of 12 plane pairs takes 19.0 us
+// (27.6 us with separate real and imaginary planes of padded rows, whose
+// scalar accesses cost twice the shared-memory instructions and 1.7 M bank
+// conflicts).
 template <int H, int CW>
-__global__ void __launch_bounds__(CW * 32, FMVD_COL_MIN_BLOCKS) col_pass_w(const ColArgs a)
+__global__ void __launch_bounds__(CW * 32, FMVD_COL_MIN_BLOCKS * (8 / CW)) col_pass_w(const ColArgs a)
 {
     using WF = WarpFft<H>;
     constexpr int T = WF::T, E = WF::E, G = 32 / T, FC = CW * G, NT = CW * 32;
-    using TL = ColTile<T, FC>;
+    using TL = ColTile<H, FC>;
     extern __shared__ __align__(16) float smem[];
-    float *tre = smem;
-    float *tim = smem + H * TL::ld;
     const int W = a.W;
     const int p = blockIdx.y;
-    const int x0 = blockIdx.x * FC;
-    float2 *C = a.C + (size_t)p * H * W + x0;
+    float2 *C = a.C + (size_t)p * H * W + blockIdx.x * FC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float2 *sp = a.spec + (size_t)(blockIdx.x * CW + warp) * E * 32 + lane;
     // this block's slice of the spectrum (contiguous in the launch layout)
     // is brought into L2 while the tile loads and the first transform runs
     pdl_launch_dependents();
     if (threadIdx.x == 0)
-        bulk_prefetch_l2(a.spec + (size_t)blockIdx.x * E * NT, (uint32_t)(E * NT * sizeof(float2)));
+        bulk_prefetch_l2(sp, (uint32_t)(E * NT * sizeof(float2)));
     pdl_wait();
 
-    if constexpr (T == 32 && FC == 8) {
-        static_assert(H == 1024, "the interleaved tile path is the 1024-point column transform");
-        // interleaved tile on a 2048-byte boundary, filled asynchronously
-        const uint32_t s0 = smem_u32addr(smem);
-        const uint32_t base = (s0 + 2047u) & ~2047u;
-        float2 *tile = reinterpret_cast<float2 *>(reinterpret_cast<char *>(smem) + (base - s0));
+    const uint32_t s0 = smem_u32addr(smem);
+    const uint32_t base = (s0 + TL::align - 1) & ~(TL::align - 1);
+    // fill: U-byte units; a thread keeps its unit of the row and steps RI
+    // rows at a time, a multiple of the rows f tells apart, so its swizzle
+    // is a constant
+    constexpr int U = TL::pairs ? 16 : 8, UR = TL::RB / U, RI = NT / UR;
+    static_assert(RI % TL::rows == 0 && H % RI == 0, "a thread's rows share one swizzle");
+    {
+        const int y = threadIdx.x / UR, u = threadIdx.x % UR;
+        const uint32_t dst = base + TL::RB * y + ((uint32_t)(U * u) ^ (8u * TL::f(y)));
+        const char *src = reinterpret_cast<const char *>(C + (size_t)y * W) + U * u;
+        const size_t pitch = (size_t)RI * W * sizeof(float2);
 #pragma unroll 8
-        for (int u = threadIdx.x; u < H * 8; u += NT) {
-            const int y = u >> 3, c = u & 7;
-            cp_async8(tile + ColTile2::at(y, c), C + (size_t)y * W + c);
+        for (int i = 0; i < H / RI; i++) {
+            if constexpr (TL::pairs)
+                cp_async16(dst + RI * TL::RB * i, src + pitch * i);
+            else
+                cp_async8(dst + RI * TL::RB * i, src + pitch * i);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        const int warp = threadIdx.x >> 5, t = threadIdx.x & 31;
-        const uint32_t q = 64u * t + 8u * (warp ^ ((t >> 1) & 7));
-        const uint32_t wbase = base | q, rbase = (base + 2048u * t) | q;
-        float2 v[E];
-#pragma unroll
-        for (int m = 0; m < E; m++)
-            v[m] = lds2(wbase + 2048u * m);  // row t + 32 m
-        const float2 *sp = a.spec + (size_t)blockIdx.x * E * NT + threadIdx.x;
-#pragma unroll 1
-        for (int pass = 0; pass < 2; pass++) {
-            col_fft_1024<-1>(v, a.tw, wbase, rbase, t);
-            if (pass == 1)
-                break;
-#pragma unroll
-            for (int m0 = 0; m0 < E; m0 += 8) {
-                asm volatile("" ::: "memory");
-#pragma unroll
-                for (int m = m0; m < m0 + 8 && m < E; m++) {
-                    const float2 z = cmul(v[m], __ldg(sp + (size_t)m * NT));
-                    v[m] = make_float2(z.x, -z.y);
-                }
-            }
-            asm volatile("" ::: "memory");
-        }
-#pragma unroll
-        for (int m = 0; m < E; m++)
-            sts2(wbase + 2048u * m, make_float2(v[m].x, -v[m].y));
-        __syncthreads();
-#pragma unroll 4
-        for (int u = threadIdx.x; u < H * 4; u += NT) {
-            const int y = u >> 2, c = 2 * (u & 3);
-            const float2 e0 = tile[ColTile2::at(y, c)], e1 = tile[ColTile2::at(y, c + 1)];
-            *reinterpret_cast<float4 *>(C + (size_t)y * W + c) = make_float4(e0.x, e0.y, e1.x, e1.y);
-        }
-        return;
     }
-
-    constexpr int units = H * FC / 2;
-#pragma unroll 4
-    for (int u = threadIdx.x; u < units; u += NT) {
-        const int c2 = u % (FC / 2), y = u / (FC / 2);
-        const float4 q = *reinterpret_cast<const float4 *>(C + (size_t)y * W + 2 * c2);
-        const int a0 = TL::at(y, 2 * c2), a1 = TL::at(y, 2 * c2 + 1);
-        tre[a0] = q.x;
-        tim[a0] = q.y;
-        tre[a1] = q.z;
-        tim[a1] = q.w;
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / T, t = lane % T;
-    const typename TL::ColumnAddr addr{warp * G + g};
+    const int t = TL::pos(lane), c = warp * G + TL::line(lane);
+    const uint32_t q = TL::RB * t + 8u * (c ^ TL::f(t));
+    uint32_t wbase = base | q, rbase = (base + TL::align * t) | q;
+    const float2 *tw = a.tw;
     float2 v[E];
 #pragma unroll
-    for (int m = 0; m < E; m++) {
-        const int q = addr(t + T * m);
-        v[m] = make_float2(tre[q], tim[q]);
-    }
+    for (int m = 0; m < E; m++)
+        v[m] = lds2(wbase + TL::align * m);  // row t + T m
     // pass 0: forward transform, times the spectrum, conjugated; pass 1: the
     // same forward code gives the conjugate of the inverse transform
-    const float2 *sp = a.spec + (size_t)blockIdx.x * E * NT + threadIdx.x;
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
-        WF::template run_addr<-1>(v, a.tw, tre, tim, t, addr);
+        // opaque per pass: addresses and twiddles are formed where they are
+        // used instead of being kept in registers across the loop
+        asm volatile("" : "+r"(wbase), "+r"(rbase), "+l"(tw));
+        col_fft<H, FC, -1>(v, tw, wbase, rbase, t);
         if (pass == 1)
             break;
 #pragma unroll
@@ -651,24 +590,29 @@ __global__ void __launch_bounds__(CW * 32, FMVD_COL_MIN_BLOCKS) col_pass_w(const
             asm volatile("" ::: "memory");
 #pragma unroll
             for (int m = m0; m < m0 + 8 && m < E; m++) {
-                const float2 z = cmul(v[m], __ldg(sp + (size_t)m * NT));
+                const float2 z = cmul(v[m], __ldg(sp + m * 32));
                 v[m] = make_float2(z.x, -z.y);
             }
         }
         asm volatile("" ::: "memory");
     }
 #pragma unroll
-    for (int m = 0; m < E; m++) {
-        const int q = addr(t + T * m);
-        tre[q] = v[m].x;
-        tim[q] = -v[m].y;
-    }
+    for (int m = 0; m < E; m++)
+        sts2(wbase + TL::align * m, make_float2(v[m].x, -v[m].y));
     __syncthreads();
+    constexpr int PR = TL::RB / 16;
 #pragma unroll 4
-    for (int u = threadIdx.x; u < units; u += NT) {
-        const int c2 = u % (FC / 2), y = u / (FC / 2);
-        const int a0 = TL::at(y, 2 * c2), a1 = TL::at(y, 2 * c2 + 1);
-        *reinterpret_cast<float4 *>(C + (size_t)y * W + 2 * c2) = make_float4(tre[a0], tim[a0], tre[a1], tim[a1]);
+    for (int n = threadIdx.x; n < H * PR; n += NT) {
+        const int y = n / PR, u = n % PR;
+        const uint32_t row = base + TL::RB * y;
+        float4 e;
+        if constexpr (TL::pairs) {
+            e = lds4(row + ((16u * u) ^ (8u * TL::f(y))));
+        } else {
+            const float2 e0 = lds2(row + ((16u * u) ^ (8u * TL::f(y)))), e1 = lds2(row + ((16u * u + 8) ^ (8u * TL::f(y))));
+            e = make_float4(e0.x, e0.y, e1.x, e1.y);
+        }
+        *reinterpret_cast<float4 *>(C + (size_t)y * W + 2 * u) = e;
     }
 }
 
@@ -739,7 +683,7 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
     // (the weight row, a plan constant, before the dependency wait)
     constexpr bool staged = SMEM && MODE != ROW_INIT;
     __shared__ __align__(8) uint64_t sbar[2];
-    const uint32_t rb = a.d.dataW * (MODE == ROW_UPDATE ? (uint32_t)sizeof(float) : (BITS == 8 ? 1u : 2u));
+    const uint32_t rb = MODE == ROW_UPDATE ? a.d.wpitch * (uint32_t)sizeof(float) : a.d.dataW * (BITS == 8 ? 1u : 2u);
     const uint32_t rs = (rb + 15) & ~15u;
     char *const st = reinterpret_cast<char *>(smem) + sizeof(float2) * 2 * R * PF2 +
                      (size_t)h * (MODE == ROW_UPDATE ? rs : 2 * rs);
@@ -833,8 +777,6 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
         if (MODE == ROW_UPDATE) {
             prefetch_l1(work.est + r * kLineM + 16 * t);
             prefetch_l1(work.est + r * kLineM + 16 * (t + 16));
-            if (!staged)
-                prefetch_l1(work.wrow + clamp_src(r * kLineM + 32 * t, a.d.dataW, a.d.bxW));
         } else if (MODE == ROW_DIVIDE && !staged) {
             const int sx = clamp_src(r * kLineM + 64 * (t & 7), a.d.dataW, a.d.bxD);
             prefetch_l1((const char *)(t < 8 ? work.src0 : work.src1) + (size_t)sx * (BITS == 8 ? 1 : 2));
@@ -933,7 +875,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
     for (int i = 0; i < 2 * H / NT; i++) {
         const int u = threadIdx.x + i * NT;
         const int y = u >> 1, c = u & 1;
-        cp_async8(tile + coltile_r(y, c), C + (size_t)y * W + c);
+        cp_async8(base + 8 * coltile_r(y, c), C + (size_t)y * W + c);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
@@ -1074,20 +1016,20 @@ __global__ void permute_spectrum_r(const float2 *__restrict__ nat, float2 *__res
     }
 }
 
-// Launch layout of the column-pass spectrum for the warp engine.
-__global__ void permute_spectrum_w(const float2 *__restrict__ nat, float2 *__restrict__ out, int H, int W, int T,
-                                   int CW, float scale)
+// Launch layout of the column-pass spectrum for the warp engine: warp w of
+// the plane, register m, lane l (see col_pass_w).
+template <int H>
+__global__ void permute_spectrum_w(const float2 *__restrict__ nat, float2 *__restrict__ out, int W, float scale)
 {
-    const int E = H / T, G = 32 / T, FC = CW * G, NT = CW * 32;
+    constexpr int T = warp_fft_lanes(H), E = H / T, G = 32 / T;
+    using TL = ColTile<H, 2 * G>;
     const size_t total = (size_t)H * W;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int tid = (int)(i % NT);
-        const int m = (int)((i / NT) % E);
-        const int bx = (int)(i / ((size_t)NT * E));
-        const int warp = tid >> 5, lane = tid & 31;
-        const int g = lane / T, t = lane % T;
-        const int n = t + T * m;
-        const int col = stored_frequency(bx * FC + warp * G + g, W);
+        const int lane = (int)(i % 32);
+        const int m = (int)((i / 32) % E);
+        const int warp = (int)(i / (32 * E));
+        const int n = TL::pos(lane) + T * m;
+        const int col = stored_frequency(warp * G + TL::line(lane), W);
         const float2 k = nat[(size_t)n * W + col];
         out[i] = make_float2(k.x * scale, k.y * scale);
     }
@@ -1152,15 +1094,20 @@ __global__ void kspec_cols(const float2 *__restrict__ A, int kH, int H, int W, c
     K[(size_t)u * W + v] = make_float2(re.s, im.s);
 }
 
-__global__ void normalize_weights_kernel(const float *__restrict__ in, float *__restrict__ out, int V, size_t n)
+// Weights normalised over views, rows wpitch apart (the floats past dataW
+// are zero and never used).
+__global__ void normalize_weights_kernel(const float *__restrict__ in, float *__restrict__ out, const RlDims d)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t n = (size_t)d.dataH * d.dataW, pitched = (size_t)d.dataH * d.wpitch;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < pitched; i += (size_t)gridDim.x * blockDim.x) {
+        const int y = (int)(i / d.wpitch), x = (int)(i % d.wpitch);
+        const size_t j = (size_t)y * d.dataW + x;
         float s = 0.f;
-        for (int v = 0; v < V; v++)
-            s += in[(size_t)v * n + i];
-        for (int v = 0; v < V; v++) {
-            const float w = in[(size_t)v * n + i];
-            out[(size_t)v * n + i] = s > 0.f ? w / s : w;
+        for (int v = 0; v < d.V && x < d.dataW; v++)
+            s += in[(size_t)v * n + j];
+        for (int v = 0; v < d.V; v++) {
+            const float w = x < d.dataW ? in[(size_t)v * n + j] : 0.f;
+            out[(size_t)v * pitched + i] = s > 0.f ? w / s : w;
         }
     }
 }
@@ -1291,85 +1238,76 @@ static void configure_smem(K kern, size_t bytes, unsigned &mask)
 
 static bool aligned16(const void *p, size_t bytes) { return ((uintptr_t)p % 16 == 0) && bytes % 16 == 0; }
 
-// Warp row-pass variant for a launch (update passes: noout when not the
-// last view; sm when the operand rows are bulk-copied into shared memory).
+// Row-pass variant for a launch: update passes per last / not last, divide
+// passes per data rows in shared memory or not.
 template <int W, int MODE, int BITS>
-static void pick_row_w(bool noout, bool sm, void (*&kern)(const RowArgs), unsigned *&m)
+static void pick_row_w(const RowArgs &a, void (*&kern)(const RowArgs), unsigned *&m)
 {
-    static unsigned mask[4] = {0, 0, 0, 0};
-    constexpr bool U = MODE == ROW_UPDATE;
-    if (noout)
-        kern = sm ? row_pass_w<W, MODE, BITS, U, true> : row_pass_w<W, MODE, BITS, U, false>;
-    else
-        kern = sm ? row_pass_w<W, MODE, BITS, false, true> : row_pass_w<W, MODE, BITS, false, false>;
-    m = &mask[(noout ? 1 : 0) + (sm ? 2 : 0)];
+    static unsigned mask[2] = {0, 0};
+    if constexpr (MODE == ROW_UPDATE) {
+        kern = a.last ? row_pass_w<W, MODE, BITS, false, true> : row_pass_w<W, MODE, BITS, true, true>;
+        m = &mask[a.last ? 1 : 0];
+    } else {
+        kern = a.bulk_data ? row_pass_w<W, MODE, BITS, false, true> : row_pass_w<W, MODE, BITS, false, false>;
+        m = &mask[a.bulk_data ? 1 : 0];
+    }
 }
 
-// Line-engine row-pass variant for a launch (per sample width; update
-// passes per last / not last).
 template <int R, int MODE, int BITS, bool DSTEP>
-static void pick_row_r_bits(bool noout, bool sm, void (*&kern)(const RowArgs), unsigned *&m)
+static void pick_row_r_bits(const RowArgs &a, void (*&kern)(const RowArgs), unsigned *&m)
 {
-    static unsigned mask[4] = {0, 0, 0, 0};
-    constexpr bool U = MODE == ROW_UPDATE;
-    if (noout)
-        kern = sm ? row_pass_r<R, MODE, BITS, U, true, DSTEP> : row_pass_r<R, MODE, BITS, U, false, DSTEP>;
-    else
-        kern = sm ? row_pass_r<R, MODE, BITS, false, true, DSTEP> : row_pass_r<R, MODE, BITS, false, false, DSTEP>;
-    m = &mask[(noout ? 1 : 0) + (sm ? 2 : 0)];
+    static unsigned mask[2] = {0, 0};
+    if constexpr (MODE == ROW_UPDATE) {
+        kern = a.last ? row_pass_r<R, MODE, BITS, false, true, DSTEP> : row_pass_r<R, MODE, BITS, true, true, DSTEP>;
+        m = &mask[a.last ? 1 : 0];
+    } else {
+        kern = a.bulk_data ? row_pass_r<R, MODE, BITS, false, true, DSTEP>
+                           : row_pass_r<R, MODE, BITS, false, false, DSTEP>;
+        m = &mask[a.bulk_data ? 1 : 0];
+    }
 }
 
-// (sm: the operand rows may be bulk-copied into shared memory)
 template <int R, int MODE, bool DSTEP>
-static void pick_row_r(const RowArgs &a, bool sm, void (*&kern)(const RowArgs), unsigned *&m)
+static void pick_row_r(const RowArgs &a, void (*&kern)(const RowArgs), unsigned *&m)
 {
     static unsigned mask0 = 0;
-    const bool noout = MODE == ROW_UPDATE && !a.last;
     if constexpr (MODE == ROW_INIT) {
         kern = row_pass_r<R, MODE, 0, false, false, DSTEP>;
         m = &mask0;
     } else if (a.d.bits == 16) {
-        pick_row_r_bits<R, MODE, 16, DSTEP>(noout, sm, kern, m);
+        pick_row_r_bits<R, MODE, 16, DSTEP>(a, kern, m);
     } else {
-        pick_row_r_bits<R, MODE, 8, DSTEP>(noout, sm, kern, m);
+        pick_row_r_bits<R, MODE, 8, DSTEP>(a, kern, m);
     }
 }
 
 template <int W, int MODE>
 static void launch_row(const RowArgs &a0, cudaStream_t s)
 {
+    RowArgs a = a0;
+    const size_t es = a.d.bits == 16 ? 2 : 1;
+    a.bulk_data = aligned16(a.b.data, a.d.dataW * es) && (a.b.view_stride * es) % 16 == 0 &&
+                  (a.b.plane_stride * es) % 16 == 0;
+    const size_t data_row = (a.d.dataW * es + 15) & ~(size_t)15;
+    // operand rows in shared memory, per line
+    const size_t operands =
+        MODE == ROW_UPDATE ? a.d.wpitch * sizeof(float) : (MODE == ROW_DIVIDE && a.bulk_data ? 2 * data_row : 0);
+    void (*kern)(const RowArgs);
+    unsigned *m;
     if constexpr (W <= 1024) {
         using WF = WarpFft<W>;
         constexpr int G = 32 / WF::T;
-        RowArgs a = a0;
-        const size_t es = a.d.bits == 16 ? 2 : 1;
-        a.bulk_data = aligned16(a.b.data, a.d.dataW * es) && (a.b.view_stride * es) % 16 == 0 &&
-                      (a.b.plane_stride * es) % 16 == 0;
-        a.bulk_weights = aligned16(a.b.weights, a.d.dataW * sizeof(float)) &&
-                         ((size_t)a.d.dataH * a.d.dataW * sizeof(float)) % 16 == 0;
-        size_t pf = 0;
-        if (MODE == ROW_UPDATE)
-            pf = a.bulk_weights ? a.d.dataW * sizeof(float) : 0;
-        else if (MODE == ROW_DIVIDE && a.bulk_data)
-            pf = 2 * ((a.d.dataW * es + 15) & ~(size_t)15);
         static_assert(WF::padded_f2 >= W, "the update pass lands the estimate row in the transpose buffer");
-        a.group_floats = WF::padded_floats + (int)(pf / sizeof(float));
+        a.group_floats = WF::padded_floats + (int)(operands / sizeof(float));
         const size_t smem = sizeof(float) * kRowWarps * G * (size_t)a.group_floats;
-        // the element-wise step is compiled for the sample width
-        // compiled per sample width, per operand rows in shared memory or
-        // not, and for the update pass per last / not last
-        void (*kern)(const RowArgs);
-        unsigned *m;
-        const bool noout = MODE == ROW_UPDATE && !a.last;
-        const bool sm = MODE == ROW_UPDATE ? a.bulk_weights != 0 : (MODE == ROW_DIVIDE && a.bulk_data != 0);
         if constexpr (MODE == ROW_INIT) {
             static unsigned mask0 = 0;
             kern = row_pass_w<W, MODE, 0, false, false>;
             m = &mask0;
         } else if (a.d.bits == 16) {
-            pick_row_w<W, MODE, 16>(noout, sm, kern, m);
+            pick_row_w<W, MODE, 16>(a, kern, m);
         } else {
-            pick_row_w<W, MODE, 8>(noout, sm, kern, m);
+            pick_row_w<W, MODE, 8>(a, kern, m);
         }
         configure_smem(kern, 200 * 1024, *m);
         dim3 grid((a.d.H + kRowWarps * G - 1) / (kRowWarps * G), a.b.npairs);
@@ -1377,24 +1315,11 @@ static void launch_row(const RowArgs &a0, cudaStream_t s)
     } else {
         constexpr int R = W / kLineM;
         static_assert(W % kLineM == 0 && R >= 3 && R <= 8, "rows above 1024 are 3..8 sub-lines of 512");
-        RowArgs a = a0;
-        const size_t es = a.d.bits == 16 ? 2 : 1;
-        a.bulk_data = aligned16(a.b.data, a.d.dataW * es) && (a.b.view_stride * es) % 16 == 0 &&
-                      (a.b.plane_stride * es) % 16 == 0;
-        a.bulk_weights = aligned16(a.b.weights, a.d.dataW * sizeof(float)) &&
-                         ((size_t)a.d.dataH * a.d.dataW * sizeof(float)) % 16 == 0;
-        const bool sm = MODE == ROW_UPDATE ? a.bulk_weights != 0 : (MODE == ROW_DIVIDE && a.bulk_data != 0);
-        size_t smem = sizeof(float2) * 2 * R * WarpFft<kLineM>::padded_f2;
-        if (sm) {
-            const size_t rs = ((size_t)a.d.dataW * (MODE == ROW_UPDATE ? sizeof(float) : es) + 15) & ~(size_t)15;
-            smem += 2 * (MODE == ROW_UPDATE ? rs : 2 * rs);
-        }
-        void (*kern)(const RowArgs);
-        unsigned *m;
+        const size_t smem = sizeof(float2) * 2 * R * WarpFft<kLineM>::padded_f2 + 2 * operands;
         if (a.d.radix_step == kRadixSums)
-            pick_row_r<R, MODE, false>(a, sm, kern, m);
+            pick_row_r<R, MODE, false>(a, kern, m);
         else
-            pick_row_r<R, MODE, true>(a, sm, kern, m);
+            pick_row_r<R, MODE, true>(a, kern, m);
         configure_smem(kern, 200 * 1024, *m);
         dim3 grid(a.d.H / 2, a.b.npairs);
         launch_pass(kern, grid, dim3(R * 32), smem, s, a);
@@ -1405,10 +1330,8 @@ static void launch_row(const RowArgs &a0, cudaStream_t s)
 template <int H, int CW>
 static void launch_col_w(const ColArgs &a, int npairs, cudaStream_t s)
 {
-    using WF = WarpFft<H>;
-    constexpr int FC = CW * (32 / WF::T);
-    // the interleaved-tile path (T = 32, 8 columns) aligns its tile to 2048 bytes
-    constexpr size_t smem = sizeof(float) * 2 * H * ColTile<WF::T, FC>::ld + (WF::T == 32 && FC == 8 ? 2048 : 0);
+    constexpr int FC = CW * (32 / warp_fft_lanes(H));
+    constexpr size_t smem = ColTile<H, FC>::bytes;
     auto kern = col_pass_w<H, CW>;
     static unsigned mask = 0;
     configure_smem(kern, smem, mask);
@@ -1453,28 +1376,40 @@ static void dispatch_row(const RowArgs &a, cudaStream_t s)
 
 void rl_init(const RlDims &d, const RlBatch &b, const RlTables &t, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, t.twW};
     dispatch_row<ROW_INIT>(a, s);
 }
 
 void rl_divide(const RlDims &d, const RlBatch &b, const RlTables &t, int view, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, t.twW};
     dispatch_row<ROW_DIVIDE>(a, s);
 }
 
 void rl_update(const RlDims &d, const RlBatch &b, const RlTables &t, int view, bool last, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, t.twW};
     dispatch_row<ROW_UPDATE>(a, s);
 }
 
 void rl_col(const RlDims &d, const RlBatch &b, const RlTables &t, const float2 *spectrum, cudaStream_t s)
 {
     ColArgs a{b.C, spectrum, t.wtwH, d.H, d.W, t.twH};
+    // Four-warp blocks where eight-warp ones would number fewer than 64:
+    // twice as many multiprocessors then share the transforms.  Ten
+    // iterations of two views (us, 4 / 8 warps): one 512 x 512 pair (32 blocks
+    // of 8 warps) 519 / 643, two 128 x 128 pairs (8) 234 / 262, two 256 x 256
+    // pairs (32) 390 / 399; but two 512 x 512 pairs (64) 865 / 814 and eight
+    // 256 x 256 pairs (128) 523 / 502.  Two warps were never best beyond noise.
+    int cw = d.col_warps;
+    if (d.col_auto && d.H <= 1024) {
+        const int G = 32 / warp_fft_lanes(d.H);
+        if (cw == 8 && d.W / (cw * G) * b.npairs < 64)
+            cw = 4;
+    }
     switch (d.H) {
 #define X(N) \
-    case N: launch_col<N>(a, b.npairs, d.col_warps ? d.col_warps : col_warps(d.H, d.W), d.radix_step, s); break;
+    case N: launch_col<N>(a, b.npairs, cw, d.radix_step, s); break;
         FMVD_FOR_EACH_LENGTH(X)
 #undef X
     default: break;
@@ -1496,7 +1431,7 @@ int rl_warp_twiddle_entries(int n)
 }
 
 void rl_kernel_spectrum(const float *d_kernel, int kH, int kW, int H, int W, const float2 *twH, const float2 *twW,
-                        float2 *work, float2 *d_out, int cw, cudaStream_t s)
+                        float2 *work, float2 *d_out, cudaStream_t s)
 {
     float2 *A = work;
     float2 *K = work + (size_t)kH * W;
@@ -1507,11 +1442,17 @@ void rl_kernel_spectrum(const float *d_kernel, int kH, int kW, int H, int W, con
     // 1 / (H W), rounded once to float (the reference's modulateAndNormalize
     // factor, fmvd_deconvolve_cuda.cu:369)
     const float scale = (float)(1.0 / ((double)H * (double)W));
-    if (H <= 1024) {
-        permute_spectrum_w<<<blocks, 256, 0, s>>>(K, d_out, H, W, warp_fft_lanes(H), cw ? cw : col_warps(H, W),
-                                                  scale);
-    } else {
-        permute_spectrum_r<<<blocks, 256, 0, s>>>(K, d_out, H, W, scale);
+    switch (H) {
+#define X(N) \
+    case N: \
+        if constexpr (N <= 1024) \
+            permute_spectrum_w<N><<<blocks, 256, 0, s>>>(K, d_out, W, scale); \
+        else \
+            permute_spectrum_r<<<blocks, 256, 0, s>>>(K, d_out, H, W, scale); \
+        break;
+        FMVD_FOR_EACH_LENGTH(X)
+#undef X
+    default: break;
     }
 }
 
@@ -1527,12 +1468,11 @@ void rl_split_estimate(const RlDims &d, const float2 *est, int nplanes, float *o
     g_launches++;
 }
 
-void rl_normalize_weights(const float *d_in, float *d_out, int V, size_t n, cudaStream_t s)
+void rl_normalize_weights(const RlDims &d, const float *d_in, float *d_out, cudaStream_t s)
 {
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 4096)
-        blocks = 4096;
-    normalize_weights_kernel<<<blocks, 256, 0, s>>>(d_in, d_out, V, n);
+    const size_t n = (size_t)d.dataH * d.wpitch;
+    const int blocks = (int)((n + 255) / 256 > 4096 ? 4096 : (n + 255) / 256);
+    normalize_weights_kernel<<<blocks, 256, 0, s>>>(d_in, d_out, d);
 }
 
 void rl_conv_same(const float *d_img, int dH, int dW, const float *d_k, int kH, int kW, float *d_out, cudaStream_t s)

@@ -18,6 +18,8 @@ struct RlDims {
     int byD, bxD;
     int byW, bxW;
     int col_warps;       // column-pass warps per block (warp engine, H <= 1024)
+    int col_auto;        // the caller left col_warps to the library: narrower blocks for few planes
+    int wpitch;          // floats per stored weight row: dataW rounded up to a multiple of 4
     int radix_step;      // lines above 1024: kRadixDft or kRadixSums
 };
 
@@ -35,7 +37,7 @@ struct RlBatch {
     const void *data;     // view v, plane z at data + (v * view_stride + z * plane_stride) samples
     size_t view_stride;
     size_t plane_stride;  // dataH * dataW
-    const float *weights; // V x dataH x dataW, normalised over views
+    const float *weights; // V x dataH x wpitch, normalised over views
     void *out;            // nplanes x dataH x dataW samples
     int npairs;
     int nplanes;
@@ -88,12 +90,12 @@ void rl_split_estimate(const RlDims &d, const float2 *est, int nplanes, float *o
 // Kernel spectrum of a kH x kW kernel centred at (kH/2, kW/2) -> (0, 0) on the
 // H x W plane, scaled by 1 / (H W), in the column-pass launch layout.
 // twH / twW: exp(-2 pi i n / N) tables; work must hold H * W + kH * W complex
-// floats.  col_warps: the plan's column-pass warps (the launch layout depends
-// on it).
+// floats.
 void rl_kernel_spectrum(const float *d_kernel, int kH, int kW, int H, int W, const float2 *twH, const float2 *twW,
-                        float2 *work, float2 *d_out, int col_warps, cudaStream_t s);
-// Weights normalised over views where the sum is positive.
-void rl_normalize_weights(const float *d_in, float *d_out, int V, size_t n, cudaStream_t s);
+                        float2 *work, float2 *d_out, cudaStream_t s);
+// Weights (V x dataH x dataW) normalised over views where the sum is
+// positive, in rows of wpitch floats.
+void rl_normalize_weights(const RlDims &d, const float *d_in, float *d_out, cudaStream_t s);
 // Clamp-to-border padded circular convolution of a dH x dW image with a
 // kH x kW kernel on the snapTransformSize domain, cropped to dH x dW.
 void rl_conv_same(const float *d_img, int dH, int dW, const float *d_k, int kH, int kW, float *d_out, cudaStream_t s);
