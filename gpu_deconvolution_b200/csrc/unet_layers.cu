@@ -99,45 +99,62 @@ __global__ void plane_scale_final_kernel(const float *parts, int N, float inv_co
 
 // col[n][y][x][k], k = t * (V + 1) + c: view c (c < V) or the views' mean
 // (c = V), divided by s[n], at (y + dy_t, x + dx_t), zero outside; k beyond
-// 9 (V + 1) zero.  A block builds kPatchPixels consecutive pixels' rows in
-// shared memory (one (pixel, tap) item per thread step, loads coalesced
-// along pixels), then writes them with 16-byte coalesced stores.
-constexpr int kPatchPixels = 128;
+// 9 (V + 1) zero.  A block makes kPatchRows x kPatchCols pixels' rows: it
+// normalises the pixels and their one-pixel surroundings once into shared
+// memory (pixel-major, V + 1 values each), where the part of a row that
+// belongs to one dy is 3 (V + 1) consecutive values, then each thread gathers
+// eight values k = 8 j .. 8 j + 7 of a pixel and writes them with one 16-byte
+// store, consecutive threads consecutive units.
+// Issue-bound (74 %): four planes of 512 x 512, four views, 43 us; one pixel
+// and tap per thread step, with 2-byte shared stores 128 bytes apart (46 M bank
+// conflicts), took 195 us.
+constexpr int kPatchRows = 8, kPatchCols = 128;
 __global__ void __launch_bounds__(256) input_patches_kernel(const unsigned short *views, size_t view_stride, int V,
-                                                            int N, int H, int W, const float *scale, bf16 *col)
+                                                            int H, int W, const float *scale, bf16 *col)
 {
-    __shared__ __align__(16) bf16 rows[kPatchPixels * kInputChannels];
-    const size_t P = (size_t)N * H * W;
-    for (size_t p0 = (size_t)blockIdx.x * kPatchPixels; p0 < P; p0 += (size_t)gridDim.x * kPatchPixels) {
-        const int np = P - p0 < (size_t)kPatchPixels ? (int)(P - p0) : kPatchPixels;
-        for (int i = threadIdx.x; i < kPatchPixels * kInputChannels / 8; i += blockDim.x)
-            reinterpret_cast<uint4 *>(rows)[i] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-        for (int item = threadIdx.x; item < 9 * kPatchPixels; item += blockDim.x) {
-            const int t = item / kPatchPixels, i = item % kPatchPixels;
-            if (i >= np)
-                continue;
-            const size_t p = p0 + i;
-            const int x = (int)(p % W), y = (int)((p / W) % H), n = (int)(p / ((size_t)W * H));
-            const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
-            if (yy < 0 || yy >= H || xx < 0 || xx >= W)
-                continue;
-            const float inv = 1.f / scale[n];
-            const size_t q = ((size_t)n * H + yy) * W + xx;
-            bf16 *r = rows + i * kInputChannels + t * (V + 1);
-            float mean = 0.f;
-            for (int c = 0; c < V; c++) {
-                const float v = (float)views[c * view_stride + q] * inv;
-                r[c] = f2b(v);
-                mean += v;
-            }
-            r[V] = f2b(mean / (float)V);
+    constexpr int TR = kPatchRows + 2, TC = kPatchCols + 2;
+    __shared__ bf16 px[TR * TC * (kInputChannels / 9)];
+    const int K = V + 1;
+    const int x0 = blockIdx.x * kPatchCols, y0 = blockIdx.y * kPatchRows, n = blockIdx.z;
+    const float inv = 1.f / scale[n];
+    for (int i = threadIdx.x; i < TR * TC; i += blockDim.x) {
+        const int yy = y0 + i / TC - 1, xx = x0 + i % TC - 1;
+        bf16 *r = px + i * K;
+        if (yy < 0 || yy >= H || xx < 0 || xx >= W) {
+            for (int c = 0; c < K; c++)
+                r[c] = f2b(0.f);
+            continue;
         }
-        __syncthreads();
-        uint4 *dst = reinterpret_cast<uint4 *>(col + p0 * kInputChannels);
-        for (int i = threadIdx.x; i < np * kInputChannels / 8; i += blockDim.x)
-            dst[i] = reinterpret_cast<const uint4 *>(rows)[i];
-        __syncthreads();
+        const size_t q = ((size_t)n * H + yy) * W + xx;
+        float mean = 0.f;
+        for (int c = 0; c < V; c++) {
+            const float v = (float)views[c * view_stride + q] * inv;
+            r[c] = f2b(v);
+            mean += v;
+        }
+        r[V] = f2b(mean / (float)V);
+    }
+    __syncthreads();
+    // this thread's eight values, as offsets from its pixel's place in px
+    // (negative: beyond 9 (V + 1))
+    constexpr int units = kInputChannels / 8;
+    const int j = threadIdx.x % units;
+    int off[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const int k = 8 * j + e, dy = k / (3 * K);
+        off[e] = k < 9 * K ? dy * TC * K + k % (3 * K) : -1;
+    }
+    const int rows = min(kPatchRows, H - y0);
+    for (int i = threadIdx.x / units; i < rows * kPatchCols; i += blockDim.x / units) {
+        const int y = i / kPatchCols, x = i % kPatchCols;
+        const bf16 *p = px + (y * TC + x) * K;
+        __align__(16) bf16 h[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            h[e] = off[e] >= 0 ? p[off[e]] : f2b(0.f);
+        reinterpret_cast<uint4 *>(col + (((size_t)n * H + y0 + y) * W + x0 + x) * kInputChannels)[j] =
+            *reinterpret_cast<const uint4 *>(h);
     }
 }
 
@@ -306,45 +323,50 @@ __global__ void output_kernel(const bf16 *act, const float *w, const float *b, i
     }
 }
 
-// g_act[p][c] = gy[p] w[c] where act > 0; dw[c] += sum_p gy[p] act[p][c]; db += sum_p gy[p]
+// g_act[p][c] = gy[p] w[c] where act > 0; dw[c] += sum_p gy[p] act[p][c]; db += sum_p gy[p].
+// Thread (row r, chunk cc) takes eight channels of pixels r, r + rows, ...;
+// the block's partial sums meet in registers (lanes of equal chunk) before one
+// shared-memory atomic per warp and channel.
+// Bound by its traffic (132 bytes per pixel): four planes of 512 x 512 take 34
+// us; with all channels per thread and 33 shared atomics by every thread 730 us.
 __global__ void output_grad_kernel(const bf16 *act, const float *w, int C, size_t P, const float *gy, bf16 *g_act,
                                    float *dw, float *db)
 {
     __shared__ float sdw[kMaxOutChannels + 1];
-    __shared__ float sw[kMaxOutChannels];
-    for (int i = threadIdx.x; i <= C; i += blockDim.x) {
+    const int C8 = C / 8, rows = blockDim.x / C8;  // C8 divides 32
+    const int cc = threadIdx.x % C8, r = threadIdx.x / C8;
+    for (int i = threadIdx.x; i <= C; i += blockDim.x)
         sdw[i] = 0.f;
-        if (i < C)
-            sw[i] = w[i];
-    }
-    __syncthreads();
-    float pdw[kMaxOutChannels];
+    float sw[8], pdw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, pdb = 0.f;
 #pragma unroll
-    for (int c = 0; c < kMaxOutChannels; c++)
-        pdw[c] = 0.f;
-    float pdb = 0.f;
-    FOR_ITEMS(p, P) {
+    for (int e = 0; e < 8; e++)
+        sw[e] = w[8 * cc + e];
+    __syncthreads();
+    for (size_t p = blockIdx.x * (size_t)rows + r; p < P; p += (size_t)gridDim.x * rows) {
         const float g = gy[p];
         pdb += g;
+        float a[8], o[8];
+        load8(act + p * C + 8 * cc, a);
 #pragma unroll
-        for (int c0 = 0; c0 < kMaxOutChannels; c0 += 8) {
-            if (c0 >= C)
-                break;
-            float a[8], o[8];
-            load8(act + p * C + c0, a);
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                pdw[c0 + e] += g * a[e];
-                o[e] = a[e] > 0.f ? g * sw[c0 + e] : 0.f;
-            }
-            store8(g_act + p * C + c0, o);
+        for (int e = 0; e < 8; e++) {
+            pdw[e] += g * a[e];
+            o[e] = a[e] > 0.f ? g * sw[e] : 0.f;
         }
+        store8(g_act + p * C + 8 * cc, o);
     }
+    for (int o = C8; o < 32; o <<= 1) {
 #pragma unroll
-    for (int c = 0; c < kMaxOutChannels; c++)
-        if (c < C)
-            atomicAdd(&sdw[c], pdw[c]);
-    atomicAdd(&sdw[C], pdb);
+        for (int e = 0; e < 8; e++)
+            pdw[e] += __shfl_xor_sync(0xffffffffu, pdw[e], o);
+        pdb += __shfl_xor_sync(0xffffffffu, pdb, o);
+    }
+    if ((threadIdx.x & 31) < C8) {
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            atomicAdd(&sdw[8 * cc + e], pdw[e]);
+        if (cc == 0)
+            atomicAdd(&sdw[C], pdb);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < C; i += blockDim.x)
         atomicAdd(dw + i, sdw[i]);
@@ -431,9 +453,8 @@ bool plane_scale(const unsigned short *views, size_t view_stride, int V, int N, 
 bool input_patches(const unsigned short *views, size_t view_stride, int V, int N, int H, int W, const float *scale,
                    bf16 *col, cudaStream_t s)
 {
-    const size_t groups = ((size_t)N * H * W + kPatchPixels - 1) / kPatchPixels;
-    input_patches_kernel<<<(int)(groups < 148 * 8 ? groups : 148 * 8), 256, 0, s>>>(views, view_stride, V, N, H, W,
-                                                                                   scale, col);
+    const dim3 grid(W / kPatchCols, (H + kPatchRows - 1) / kPatchRows, N);  // W is a multiple of 128 (create)
+    input_patches_kernel<<<grid, 256, 0, s>>>(views, view_stride, V, H, W, scale, col);
     rl_count_launch(1);
     return FMVD_CHECK(cudaGetLastError());
 }
@@ -490,7 +511,8 @@ bool output_layer(const bf16 *act, const float *w, const float *b, int C, int N,
 bool output_grad(const bf16 *act, const float *w, int C, size_t P, const float *gy, bf16 *g_act, float *dw,
                  float *db, cudaStream_t s)
 {
-    output_grad_kernel<<<grid_for(P), 256, 0, s>>>(act, w, C, P, gy, g_act, dw, db);
+    const size_t need = (P + 256 / (C / 8) - 1) / (256 / (C / 8));
+    output_grad_kernel<<<(int)(need < 148 * 8 ? need : 148 * 8), 256, 0, s>>>(act, w, C, P, gy, g_act, dw, db);
     rl_count_launch(1);
     return FMVD_CHECK(cudaGetLastError());
 }
