@@ -25,17 +25,17 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)
 __host__ __device__ constexpr uint32_t layout_code(int row_bytes) { return row_bytes == 128 ? 2u : 4u; }
 
 // Shared-memory matrix descriptor (version 1, base offset 0, legacy LBO
-// mode): start, leading and stride byte offsets in 16-byte units.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes,
-                                              int row_bytes)
+// mode): start, leading and stride byte offsets in 16-byte units.  Kept as two
+// words: the start address (below 256 KB, so it never carries out of its
+// field) is in the lower one, and moving an operand by b bytes adds b / 16.
+struct Desc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc operator+(uint32_t bytes) const { return Desc{lo + bytes / 16, hi}; }
+};
+__device__ __forceinline__ Desc make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, int row_bytes)
 {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1u << 46;  // descriptor version for sm_100
-    d |= (uint64_t)layout_code(row_bytes) << 61;
-    return d;
+    return Desc{(saddr >> 4) | ((lbo_bytes >> 4) << 16),
+                (sbo_bytes >> 4) | (1u << 14) /* descriptor version for sm_100 */ | (layout_code(row_bytes) << 29)};
 }
 
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 accumulator,
@@ -69,22 +69,45 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// ---- MMA (one thread) -------------------------------------------------------
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate)
+// ---- MMA (a whole, converged warp; an elected lane issues) -------------------
+// The role's code runs on every lane, so that descriptors and addresses stay
+// warp-uniform, and elect.sync picks the lane that issues.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, Desc a, Desc b, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem_d),
+        "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// The mbarrier receives one arrival when every MMA this thread issued
-// before has completed (and released its shared-memory operands).
+// The mbarrier receives one arrival when every MMA the elected lane issued before
+// has completed (and released its shared-memory operands).
 __device__ __forceinline__ void mma_commit(uint64_t *bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
+        : "memory");
+}
+// This thread's warp, as a value the compiler knows to be the same on all lanes.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// ---- 32-byte global accesses (p on a 32-byte boundary) -----------------------
+__device__ __forceinline__ void ldg32(const void *p, uint32_t (&r)[8])
+{
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void stg32(void *p, const uint32_t (&r)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
 

@@ -11,11 +11,11 @@ namespace unet {
 // Kernel arguments of the convolution GEMM (see unet_gemm.cu).
 struct GemmArgs {
     int N, H, W;          // images and image size of the pixel grid
-    int bw, bh;           // pixel box of one tile (mode 0) or K block (mode 1)
+    int bw, bh;           // pixel box of one tile (conv_gemm_persistent)
     int taps;             // 9 (3 x 3) or 1
     int cin, cout;        // channels of the input / output of the convolution
-    int kchunk;           // mode 1: pixel K blocks per CTA
-    __nv_bfloat16 *out;   // mode 0 outputs
+    int vec;              // bias, add, mask and out may be accessed 32 bytes at a time
+    __nv_bfloat16 *out;   // forward outputs
     int out_ld, out_coff;
     float *out_f32;
     int outf_ld;
@@ -25,7 +25,8 @@ struct GemmArgs {
     const __nv_bfloat16 *mask;
     int mask_ld;
     int relu;
-    float *dw;            // mode 1 output, [cout][taps][cin], accumulated
+    float *dw;            // weight-gradient output, [cout][taps][cin], accumulated
+    float *db;            // bias-gradient output, [cout], accumulated, or null
     int *status;          // set to 1 when a wait timed out
 };
 
@@ -51,11 +52,12 @@ struct ConvDesc {
 };
 
 // dw[co][t][ci] += sum_{n, y, x} grad[n][y][x][co] * in[n][y + dy_t][x + dx_t][ci]
+// and, unless null, db[co] += sum_{n, y, x} grad[n][y][x][co]
 struct WgradDesc {
     const __nv_bfloat16 *grad;
     const __nv_bfloat16 *in;
     int N, H, W, cin, cout, taps;
-    float *dw;
+    float *dw, *db;
     int *status;
 };
 

@@ -1,27 +1,29 @@
 // BF16 implicit-GEMM 3x3 / 1x1 convolutions on the tcgen05 tensor cores
 // (FP32 accumulation in tensor memory), for the warm-start network.
 //
-// Activations are NHWC bf16; weights [Cout][taps][Cin] bf16.  Two GEMM forms:
+// Activations are NHWC bf16; weights [Cout][taps][Cin] bf16.
 //
-//   mode 0 (forward and data gradient): D[pixel][co] = sum over taps t and
-//     input channels ci of A[pixel + off(t)][ci] * B[co][t][ci].  A tile is
-//     128 output pixels (a bw x bh patch of one image); each K block is one
-//     tap and CB input channels, loaded by a 4-D TMA box whose out-of-image
-//     part arrives as zeros (the convolution's zero padding).  Both operands
-//     are K-major.  The epilogue adds the bias and an optional skip tensor,
-//     applies ReLU, zeroes where a mask tensor is <= 0 (the ReLU derivative
-//     of the data gradient) and stores bf16 (and/or fp32).
-//   mode 1 (weight gradient): D[co][ci] = sum over pixels p of
-//     G[p][co] * X[p + off(t)][ci] for one tap t.  K runs over pixels, so
-//     both operands are MN-major (channels contiguous); the pixel range is
-//     split over CTAs and the FP32 partial sums are added into dW with
+//   conv_halo (3x3 forward and data gradient, narrow layers) and
+//   conv_gemm_persistent (every other forward): D[pixel][co] = sum over taps t
+//     and input channels ci of A[pixel + off(t)][ci] * B[co][t][ci], taps
+//     outermost, so both give the same sums.  Both operands are K-major.  The
+//     epilogue adds the bias and an optional skip tensor, applies ReLU, zeroes
+//     where a mask tensor is <= 0 (the ReLU derivative of the data gradient)
+//     and stores bf16 (and/or fp32).
+//   conv_wgrad_kernel (weight and bias gradient): D[ci][co] = sum over pixels
+//     p of X[p + off(t)][ci] * G[p][co], all taps in one CTA.  K runs over
+//     pixels, so both operands are MN-major (channels contiguous); the pixels
+//     are split over CTAs and the FP32 partial sums are added into dW with
 //     atomics.
 //
-// One CTA of 4 warps computes a 128 x BN tile: warp 0 lane 0 issues the TMA
-// loads into a ring of shared-memory stages, warp 1 lane 0 issues the MMAs
-// and commits each stage back to the producer, then all warps read the
-// accumulator from tensor memory.  Every mbarrier wait is bounded: on a
-// timeout the CTA records an error in *status and finishes without hanging.
+// Tiles come in by 4-D TMA boxes whose out-of-image part arrives as zeros
+// (the convolution's zero padding).  The swizzle of a staged box is a
+// function of the shared-memory address alone, so an operand may start at any
+// of its pixels: the nine taps of a tile are nine start addresses into one
+// box with a one-pixel border.
+//
+// Every mbarrier wait is bounded: on a timeout the CTA records an error in
+// *status and finishes without hanging.
 #include "fmvd_internal.h"
 #include "tma_util.cuh"
 #include "umma.cuh"
@@ -29,29 +31,13 @@
 
 #include <cuda_bf16.h>
 #include <stdio.h>
+#include <algorithm>
 
 namespace fmvd {
 namespace unet {
 
 using bf16 = __nv_bfloat16;
-constexpr int kKP = 64;  // pixels per K block of the weight gradient
-
 __host__ __device__ constexpr uint32_t align1k(uint32_t b) { return (b + 1023u) & ~1023u; }
-
-template <int MODE, int CBA, int CBB, int BN>
-struct GemmCfg {
-    static constexpr int RA = CBA * 2, RB = CBB * 2;  // bytes per staged row
-    static constexpr uint32_t SA = MODE == 0 ? 128u * RA : (uint32_t)kKP * 128u * 2u;
-    static constexpr uint32_t SB = MODE == 0 ? (uint32_t)BN * RB : (uint32_t)kKP * BN * 2u;
-    static constexpr uint32_t SA_AL = align1k(SA), SB_AL = align1k(SB);
-    static constexpr uint32_t STAGE = SA_AL + SB_AL;
-    static constexpr int STAGES = 98304u / STAGE >= 4 ? 4 : (98304u / STAGE >= 2 ? (int)(98304u / STAGE) : 2);
-    static constexpr uint32_t SMEM = STAGES * STAGE + 1024;
-    static constexpr int TCOLS = BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
-    static constexpr int KSTEPS = MODE == 0 ? CBA / 16 : kKP / 16;
-    static_assert(MODE == 1 || CBA == CBB, "forward K blocks share one channel block");
-    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "N tile");
-};
 
 __device__ __forceinline__ void tap_offset(int taps, int t, int &dy, int &dx)
 {
@@ -63,195 +49,85 @@ __device__ __forceinline__ void tap_offset(int taps, int t, int &dy, int &dx)
     }
 }
 
-template <int MODE, int CBA, int CBB, int BN>
-__global__ void __launch_bounds__(128, 1)
-    conv_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g)
+// Sixteen bf16 values as floats (vec: p on a 32-byte boundary).
+__device__ __forceinline__ void load16(const bf16 *p, int vec, float (&f)[16])
 {
-    using C = GemmCfg<MODE, CBA, CBB, BN>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t *sa = smem;
-    uint8_t *sb = smem + C::STAGES * C::SA_AL;
-    __shared__ __align__(8) uint64_t full[C::STAGES], empty[C::STAGES], done;
-    __shared__ uint32_t tmem_sh;
-    __shared__ int fail_sh;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    // ---- tile coordinates
-    int n = 0, y0 = 0, x0 = 0, co0 = 0, ci0 = 0, tap = 0, kb0 = 0, nk = 0;
-    if (MODE == 0) {
-        const int tx = g.W / g.bw, ty = g.H / g.bh;
-        const int tile = blockIdx.x;
-        n = tile / (tx * ty);
-        const int r = tile % (tx * ty);
-        y0 = (r / tx) * g.bh;
-        x0 = (r % tx) * g.bw;
-        co0 = blockIdx.y * BN;
-        nk = g.taps * (g.cin / CBA);
-    } else {
-        tap = blockIdx.x % g.taps;
-        co0 = (blockIdx.x / g.taps) * 128;
-        ci0 = blockIdx.z * BN;
-        const int total = (int)(((long long)g.N * g.H * g.W) / kKP);
-        kb0 = blockIdx.y * g.kchunk;
-        nk = min(g.kchunk, total - kb0);
-    }
-    // weight-gradient A groups that hold output channels (the rest stay zero)
-    const int ga_valid = MODE == 1 ? min(128 / CBA, (g.cout - co0 + CBA - 1) / CBA) : 0;
-
-    if (MODE == 1 && ga_valid < 128 / CBA) {
-        const int zero_from = ga_valid * kKP * C::RA;
-        for (int s = 0; s < C::STAGES; s++)
-            for (int i = zero_from / 16 + threadIdx.x; i < (int)(C::SA / 16); i += blockDim.x)
-                reinterpret_cast<uint4 *>(sa + s * C::SA_AL)[i] = make_uint4(0, 0, 0, 0);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; s++) {
-            umma::bar_init(&full[s], 1);
-            umma::bar_init(&empty[s], 1);
-        }
-        umma::bar_init(&done, 1);
-        umma::bar_fence_init();
-        fail_sh = 0;
-    }
-    if (warp == 0) {
-        umma::tmem_alloc(&tmem_sh, C::TCOLS);
-        umma::tmem_relinquish();
-    }
-    umma::tc_fence_before();
-    __syncthreads();
-    umma::tc_fence_after();
-    const uint32_t tmem = tmem_sh;
-
-    if (warp == 0 && lane == 0) {
-        // ---- producer: TMA loads of the K blocks into the stage ring
-        const uint32_t bytes = MODE == 0 ? C::SA + C::SB
-                                         : (uint32_t)ga_valid * kKP * C::RA + (uint32_t)kKP * BN * 2u;
-        for (int kb = 0; kb < nk; kb++) {
-            const int s = kb % C::STAGES, round = kb / C::STAGES;
-            if (round > 0 && !umma::bar_wait(&empty[s], (round - 1) & 1)) {
-                fail_sh = 1;
-                break;
-            }
-            umma::bar_expect_tx(&full[s], bytes);
-            uint8_t *a = sa + s * C::SA_AL;
-            uint8_t *b = sb + s * C::SB_AL;
-            if (MODE == 0) {
-                const int cblocks = g.cin / CBA;
-                const int t = kb / cblocks, cb = kb % cblocks;
-                int dy, dx;
-                tap_offset(g.taps, t, dy, dx);
-                umma::tma_load_4d(a, &tmA, cb * CBA, x0 + dx, y0 + dy, n, &full[s]);
-                umma::tma_load_2d(b, &tmB, kb * CBA, co0, &full[s]);
-            } else {
-                const long long p0 = (long long)(kb0 + kb) * kKP;
-                const int hw = g.H * g.W;
-                const int pn = (int)(p0 / hw), pr = (int)(p0 % hw);
-                const int py = pr / g.W, px = pr % g.W;
-                int dy, dx;
-                tap_offset(g.taps, tap, dy, dx);
-                for (int j = 0; j < ga_valid; j++)
-                    umma::tma_load_4d(a + j * kKP * C::RA, &tmA, co0 + j * CBA, px, py, pn, &full[s]);
-                for (int j = 0; j < BN / CBB; j++)
-                    umma::tma_load_4d(b + j * kKP * C::RB, &tmB, ci0 + j * CBB, px + dx, py + dy, pn, &full[s]);
-            }
-        }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issue
-        const uint32_t idesc = umma::make_idesc(128, BN, MODE, MODE);
-        for (int kb = 0; kb < nk; kb++) {
-            const int s = kb % C::STAGES, round = kb / C::STAGES;
-            if (!umma::bar_wait(&full[s], round & 1)) {
-                fail_sh = 1;
-                break;
-            }
-            umma::tc_fence_after();
-            const uint32_t a0 = umma::smem_addr(sa + s * C::SA_AL);
-            const uint32_t b0 = umma::smem_addr(sb + s * C::SB_AL);
+    if (vec) {
+        uint32_t w[8];
+        umma::ldg32(p, w);
 #pragma unroll
-            for (int kk = 0; kk < C::KSTEPS; kk++) {
-                uint64_t ad, bd;
-                if (MODE == 0) {
-                    ad = umma::make_desc(a0 + kk * 32, 16, 8 * C::RA, C::RA);
-                    bd = umma::make_desc(b0 + kk * 32, 16, 8 * C::RB, C::RB);
-                } else {
-                    ad = umma::make_desc(a0 + kk * 16 * C::RA, kKP * C::RA, 8 * C::RA, C::RA);
-                    bd = umma::make_desc(b0 + kk * 16 * C::RB, kKP * C::RB, 8 * C::RB, C::RB);
-                }
-                umma::mma_bf16(tmem, ad, bd, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            }
-            umma::mma_commit(&empty[s]);
-        }
-        umma::mma_commit(&done);
-    }
-    __syncwarp();
-
-    // ---- epilogue: accumulator rows are TMEM lanes (warp w: lanes 32w..)
-    const bool got = umma::bar_wait(&done, 0);
-    umma::tc_fence_after();
-    const int row = warp * 32 + lane;
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    if (MODE == 0) {
-        const int y = y0 + row / g.bw, x = x0 + row % g.bw;
-        const size_t pix = ((size_t)n * g.H + y) * g.W + x;
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-            float v[16];
-            umma::tmem_ld16(trow + c0, v);
-            const int co = co0 + c0;
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                float t = v[i];
-                if (g.bias)
-                    t += g.bias[co + i];
-                if (g.add)
-                    t += __bfloat162float(g.add[pix * g.add_ld + co + i]);
-                if (g.relu)
-                    t = fmaxf(t, 0.f);
-                if (g.mask && !(__bfloat162float(g.mask[pix * g.mask_ld + co + i]) > 0.f))
-                    t = 0.f;
-                v[i] = t;
-            }
-            if (g.out) {
-                __align__(16) bf16 h[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    h[i] = __float2bfloat16_rn(v[i]);
-                uint4 *dst = reinterpret_cast<uint4 *>(g.out + pix * g.out_ld + g.out_coff + co);
-                dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-                dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-            }
-            if (g.out_f32) {
-                float4 *dst = reinterpret_cast<float4 *>(g.out_f32 + pix * g.outf_ld + co);
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            }
+        for (int i = 0; i < 8; i++) {
+            f[2 * i] = __uint_as_float(w[i] << 16);
+            f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
         }
     } else {
-        const int co = co0 + row;
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-            float v[16];
-            umma::tmem_ld16(trow + c0, v);
-            if (co < g.cout) {
-                float *dst = g.dw + ((size_t)co * g.taps + tap) * g.cin + ci0 + c0;
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    atomicAdd(dst + i, v[i]);
-            }
-        }
+        for (int i = 0; i < 16; i++)
+            f[i] = __bfloat162float(p[i]);
     }
-    if (threadIdx.x == 0 && (!got || fail_sh) && g.status)
-        atomicExch(g.status, 1);
-    umma::tc_fence_before();
-    __syncthreads();
-    if (warp == 0)
-        umma::tmem_dealloc(tmem, C::TCOLS);
 }
 
-// Persistent forward / data-gradient GEMM (mode 0 geometry).  Each CTA
+// Epilogue of sixteen accumulator columns co.. of pixel pix: bias, skip
+// tensor, ReLU, mask, stores.  g.vec: every tensor may be accessed 32 bytes
+// (whole sectors) at a time.
+__device__ __forceinline__ void epilogue16(const GemmArgs &g, size_t pix, int co, float (&v)[16])
+{
+    float t[16];
+    if (g.bias) {
+        if (g.vec) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<float4 *>(t + 4 * i) = __ldg(reinterpret_cast<const float4 *>(g.bias + co) + i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                t[i] = g.bias[co + i];
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            v[i] += t[i];
+    }
+    if (g.add) {
+        load16(g.add + pix * g.add_ld + co, g.vec, t);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            v[i] += t[i];
+    }
+    if (g.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            v[i] = fmaxf(v[i], 0.f);
+    }
+    if (g.mask) {
+        load16(g.mask + pix * g.mask_ld + co, g.vec, t);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            v[i] = t[i] > 0.f ? v[i] : 0.f;
+    }
+    if (g.out) {
+        uint32_t h[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            h[i] = *reinterpret_cast<const uint32_t *>(&b);
+        }
+        bf16 *dst = g.out + pix * g.out_ld + g.out_coff + co;
+        if (g.vec) {
+            umma::stg32(dst, h);
+        } else {
+            reinterpret_cast<uint4 *>(dst)[0] = make_uint4(h[0], h[1], h[2], h[3]);
+            reinterpret_cast<uint4 *>(dst)[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        }
+    }
+    if (g.out_f32) {
+        float4 *dst = reinterpret_cast<float4 *>(g.out_f32 + pix * g.outf_ld + co);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+}
+
+// Persistent forward / data-gradient GEMM.  Each CTA
 // walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the 128-pixel x BN
 // output; the K blocks of consecutive tiles flow through one TMA stage ring
 // without a break, and the accumulator is double-buffered in tensor memory,
@@ -288,7 +164,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
     __shared__ uint32_t tmem_sh;
     __shared__ int fail_store;
     volatile int &fail_sh = fail_store;  // set by any role that gave up waiting
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = umma::warp_index(), lane = threadIdx.x & 31;
     const int tx = g.W / g.bw, ty = g.H / g.bh;
     const int nk = g.taps * (g.cin / CB);
     const int cblocks = g.cin / CB;
@@ -348,37 +224,33 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {
-            // ---- MMA issue
-            const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
-            int gk = 0, it = 0;
-            for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
-                const int ab = it & 1;
-                if (it >= 2 && !umma::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+        // ---- MMA issue
+        const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
+        int gk = 0, it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
+            const int ab = it & 1;
+            if (it >= 2 && !umma::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            umma::tc_fence_after();
+            const uint32_t acc = tmem + ab * C::ACC_COLS;
+            for (int kb = 0; kb < nk; kb++, gk++) {
+                const int s = gk % C::STAGES, round = gk / C::STAGES;
+                if (!umma::bar_wait(&full[s], round & 1)) {
                     fail_sh = 1;
                     break;
                 }
                 umma::tc_fence_after();
-                const uint32_t acc = tmem + ab * C::ACC_COLS;
-                for (int kb = 0; kb < nk; kb++, gk++) {
-                    const int s = gk % C::STAGES, round = gk / C::STAGES;
-                    if (!umma::bar_wait(&full[s], round & 1)) {
-                        fail_sh = 1;
-                        break;
-                    }
-                    umma::tc_fence_after();
-                    const uint32_t a0 = umma::smem_addr(smem + s * C::STAGE);
-                    const uint32_t b0 = a0 + align1k(C::SA);
+                const uint32_t a0 = umma::smem_addr(smem) + s * C::STAGE;
+                const umma::Desc ad = umma::make_desc(a0, 16, 8 * C::R, C::R);
+                const umma::Desc bd = umma::make_desc(a0 + align1k(C::SA), 16, 8 * C::R, C::R);
 #pragma unroll
-                    for (int kk = 0; kk < C::KSTEPS; kk++) {
-                        const uint64_t ad = umma::make_desc(a0 + kk * 32, 16, 8 * C::R, C::R);
-                        const uint64_t bd = umma::make_desc(b0 + kk * 32, 16, 8 * C::R, C::R);
-                        umma::mma_bf16(acc, ad, bd, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-                    }
-                    umma::mma_commit(&empty[s]);
-                }
-                umma::mma_commit(&acc_full[ab]);
+                for (int kk = 0; kk < C::KSTEPS; kk++)
+                    umma::mma_bf16(acc, ad + kk * 32, bd + kk * 32, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                umma::mma_commit(&empty[s]);
             }
+            umma::mma_commit(&acc_full[ab]);
         }
     } else {
         // ---- epilogue: warp w owns accumulator rows 32w..32w+31
@@ -400,35 +272,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 float v[16];
                 umma::tmem_ld16(trow + c0, v);
-                const int co = co0 + c0;
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    float t = v[i];
-                    if (g.bias)
-                        t += g.bias[co + i];
-                    if (g.add)
-                        t += __bfloat162float(g.add[pix * g.add_ld + co + i]);
-                    if (g.relu)
-                        t = fmaxf(t, 0.f);
-                    if (g.mask && !(__bfloat162float(g.mask[pix * g.mask_ld + co + i]) > 0.f))
-                        t = 0.f;
-                    v[i] = t;
-                }
-                if (g.out) {
-                    __align__(16) bf16 h[16];
-#pragma unroll
-                    for (int i = 0; i < 16; i++)
-                        h[i] = __float2bfloat16_rn(v[i]);
-                    uint4 *dst = reinterpret_cast<uint4 *>(g.out + pix * g.out_ld + g.out_coff + co);
-                    dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-                    dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-                }
-                if (g.out_f32) {
-                    float4 *dst = reinterpret_cast<float4 *>(g.out_f32 + pix * g.outf_ld + co);
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                }
+                epilogue16(g, pix, co0 + c0, v);
             }
             umma::tc_fence_before();
             __syncwarp();
@@ -445,6 +289,383 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         umma::tc_fence_after();
         umma::tmem_dealloc(tmem, C::TCOLS);
     }
+}
+
+// 3x3 forward / data-gradient GEMM of the narrow layers (cin = CB * NB up to
+// 128, cout = BN up to 128 with the weights within shared memory).  A tile is
+// 8 x 16 pixels; its input comes in once, with a one-pixel border (10 x 18
+// pixels per channel block), and the nine taps read it at nine start
+// addresses: 128 output pixels load 180 pixels instead of 9 x 128, and the
+// weights are loaded once per CTA.  An 8-row group of the A operand is one
+// row of the tile, so the group stride is the border box's row pitch.  Roles
+// as in conv_gemm_persistent.
+// Four 512 x 512 planes: 32 -> 32 channels 39 us (one CTA per tile and every
+// tap loaded on its own: 91 us), 64 -> 32 77 us; 64 -> 64 at 256 x 256 33 us
+// (45 us).  What bounds it: loads, stores and their latencies (with one tap
+// instead of nine the network's forward pass is 6 % faster, without the stores
+// 14 %).
+constexpr int kTileW = 8, kTileH = 16, kBoxW = kTileW + 2, kBoxH = kTileH + 2;
+constexpr uint32_t kSmemOne = 226u * 1024u, kSmemTwo = 113u * 1024u;  // per CTA, one or two CTAs on an SM
+
+template <int CB, int NB, int BN>
+struct HaloCfg {
+    static constexpr uint32_t R = CB * 2;
+    static constexpr uint32_t BOX = kBoxW * kBoxH * R, SLOT = align1k(BOX);
+    static constexpr uint32_t WB = align1k((uint32_t)BN * R), WEIGHTS = 9u * NB * WB;
+    static constexpr uint32_t BUDGET = (WEIGHTS + (NB + 1) * SLOT + 1024u <= kSmemTwo ? kSmemTwo : kSmemOne) - 1024u;
+    static constexpr int FIT = (int)((BUDGET - WEIGHTS) / SLOT);
+    static constexpr int SLOTS = FIT < 2 * NB + 2 ? FIT : 2 * NB + 2;
+    static constexpr uint32_t SMEM = WEIGHTS + SLOTS * SLOT + 1024;
+    static constexpr int ACC_COLS = BN <= 32 ? 32 : (BN <= 64 ? 64 : 128);
+    static constexpr int TCOLS = 2 * ACC_COLS;
+    static_assert(SLOTS >= NB + 1, "a tile's channel blocks and the next one's first are in flight");
+};
+
+template <int CB, int NB, int BN>
+__global__ void __launch_bounds__(kPersistentThreads, 1)
+    conv_halo(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
+              int ntiles)
+{
+    using C = HaloCfg<CB, NB, BN>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *wsm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *slots = wsm + C::WEIGHTS;
+    __shared__ __align__(8) uint64_t wfull, full[C::SLOTS], empty[C::SLOTS], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_sh;
+    __shared__ int fail_store;
+    volatile int &fail_sh = fail_store;  // set by any role that gave up waiting
+    const int warp = umma::warp_index(), lane = threadIdx.x & 31;
+    const int tx = g.W / kTileW, ty = (g.H + kTileH - 1) / kTileH;
+
+    if (threadIdx.x == 0) {
+        umma::bar_init(&wfull, 1);
+        for (int i = 0; i < C::SLOTS; i++) {
+            umma::bar_init(&full[i], 1);
+            umma::bar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            umma::bar_init(&acc_full[i], 1);
+            umma::bar_init(&acc_empty[i], 4);  // one arrival per epilogue warp
+        }
+        umma::bar_fence_init();
+        fail_sh = 0;
+    }
+    if (warp == 4) {
+        umma::tmem_alloc(&tmem_sh, C::TCOLS);
+        umma::tmem_relinquish();
+    }
+    umma::tc_fence_before();
+    __syncthreads();
+    umma::tc_fence_after();
+    const uint32_t tmem = tmem_sh;
+
+    auto tile_coords = [&](int tile, int &n, int &y0, int &x0) {
+        n = tile / (tx * ty);
+        const int r = tile % (tx * ty);
+        y0 = (r / tx) * kTileH;
+        x0 = (r % tx) * kTileW;
+    };
+
+    if (warp == 4) {
+        if (lane == 0) {
+            // ---- producer: the weights once, then the tiles' input boxes
+            umma::bar_expect_tx(&wfull, 9u * NB * BN * C::R);
+            for (int k = 0; k < 9 * NB; k++)
+                umma::tma_load_2d(wsm + k * C::WB, &tmB, k * CB, 0, &wfull);
+            int gs = 0;
+            for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x) {
+                int n, y0, x0;
+                tile_coords(tile, n, y0, x0);
+                for (int cb = 0; cb < NB; cb++, gs++) {
+                    const int s = gs % C::SLOTS, round = gs / C::SLOTS;
+                    if (round > 0 && !umma::bar_wait(&empty[s], (round - 1) & 1)) {
+                        fail_sh = 1;
+                        break;
+                    }
+                    umma::bar_expect_tx(&full[s], C::BOX);
+                    umma::tma_load_4d(slots + s * C::SLOT, &tmA, cb * CB, x0 - 1, y0 - 1, n, &full[s]);
+                }
+            }
+        }
+    } else if (warp == 5) {
+        // ---- MMA issue
+        const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
+        const umma::Desc bd = umma::make_desc(umma::smem_addr(wsm), 16, 8 * C::R, C::R);
+        if (!umma::bar_wait(&wfull, 0))
+            fail_sh = 1;
+        int gs = 0, it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++, gs += NB) {
+            const int ab = it & 1;
+            if (it >= 2 && !umma::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            const uint32_t acc = tmem + ab * C::ACC_COLS;
+            umma::Desc ad[NB];
+            bool ok = true;
+#pragma unroll
+            for (int cb = 0; cb < NB; cb++) {
+                const int s = (gs + cb) % C::SLOTS, round = (gs + cb) / C::SLOTS;
+                ok = ok && umma::bar_wait(&full[s], round & 1);
+                ad[cb] = umma::make_desc(umma::smem_addr(slots) + s * C::SLOT, 16, kBoxW * C::R, C::R);
+            }
+            if (!ok) {
+                fail_sh = 1;
+                break;
+            }
+            umma::tc_fence_after();
+#pragma unroll
+            for (int t = 0; t < 9; t++)
+#pragma unroll
+                for (int cb = 0; cb < NB; cb++)
+#pragma unroll
+                    for (int kk = 0; kk < CB / 16; kk++)
+                        umma::mma_bf16(acc, ad[cb] + (((t / 3) * kBoxW + t % 3) * C::R + kk * 32),
+                                       bd + ((t * NB + cb) * C::WB + kk * 32), idesc,
+                                       (t > 0 || cb > 0 || kk > 0) ? 1u : 0u);
+#pragma unroll
+            for (int cb = 0; cb < NB; cb++)
+                umma::mma_commit(&empty[(gs + cb) % C::SLOTS]);
+            umma::mma_commit(&acc_full[ab]);
+        }
+    } else {
+        // ---- epilogue: warp w owns accumulator rows 32w..32w+31
+        const int row = warp * 32 + lane;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
+            const int ab = it & 1;
+            if (!umma::bar_wait(&acc_full[ab], (it >> 1) & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            umma::tc_fence_after();
+            int n, y0, x0;
+            tile_coords(tile, n, y0, x0);
+            const int y = y0 + row / kTileW, x = x0 + row % kTileW;
+            const size_t pix = ((size_t)n * g.H + y) * g.W + x;
+            const uint32_t trow = tmem + ab * C::ACC_COLS + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                float v[16];
+                umma::tmem_ld16(trow + c0, v);
+                if (y < g.H)
+                    epilogue16(g, pix, c0, v);
+            }
+            umma::tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                umma::bar_arrive(&acc_empty[ab]);
+        }
+    }
+    __syncwarp();
+    umma::tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && fail_sh && g.status)
+        atomicExch(g.status, 1);
+    if (warp == 4) {
+        umma::tc_fence_after();
+        umma::tmem_dealloc(tmem, C::TCOLS);
+    }
+}
+
+// Weight and bias gradient: D[ci][co] = sum over pixels p of
+// X[p + off(t)][ci] G[p][co] for every tap t of a 128 x BN tile of (ci, co),
+// over this CTA's share of the pixels.  A tile is 16 x 8 pixels; X comes in
+// with a one-pixel border (18 x 10) and the taps are start addresses into it,
+// so X and G are loaded once instead of once per tap.  M = 128 rows are
+//   cin >= 128: 128 channels (two 64-channel groups), one tap per MMA;
+//   cin = 64:   64 channels at two neighbouring pixels (PACK = 2), the taps
+//               dx = -1, 0 of a row in one MMA and dx = 1 in a second;
+//   cin = 32:   32 channels at four neighbouring pixels (PACK = 4), the three
+//               taps of a row in one MMA.
+// The neighbouring pixel is one row of the staged box further: the M-group
+// stride of the operand's descriptor.  Rows beyond dx = 1 are not read back.
+// Warp 0 issues the TMA ring, warp 1 the MMAs; warps 2 and 3 sum the staged G
+// for the bias gradient; at the end all four read tensor memory and add the
+// sums with atomics, consecutive lanes consecutive ci.
+// The tensor cores' FP32 accumulation rounds towards zero: a sum of n pixels
+// comes out about 1.2e-9 n too small (3.7e-5 over 31.9 k pixels), so the share
+// of a CTA is bounded (launch_wgrad), and the bias
+// sums, which cancel more, are ordinary FP32 additions (as an MMA with a
+// matrix of ones they were 4.7e-5 off).
+// Four 512 x 512 planes: 32 -> 32 channels 69 us (280 us with one tap per CTA),
+// 64 -> 32 112 us (288); 64 -> 64 at 256 x 256 41 us (106); 128 -> 128 at 128 x
+// 128 53 us (98); the bias sums are part of it (they were passes of their own
+// over G).  What bounds it: the MMAs (about 90 cycles each, few CTAs).
+constexpr int kGradW = 16, kGradH = 8;
+
+template <int CB, int GROUPS, int PACK, int BN, int TAPS>
+struct WgradCfg {
+    static constexpr int NACC = TAPS == 1 ? 1 : PACK == 4 ? 3 : PACK == 2 ? 6 : 9;
+    static constexpr int XW = TAPS == 1 ? kGradW : kGradW + 2, XH = TAPS == 1 ? kGradH : kGradH + 2;
+    static constexpr uint32_t R = CB * 2, XBOX = XW * XH * R, XS = align1k(XBOX);
+    static constexpr int CBG = BN >= 64 ? 64 : 32, NG = BN / CBG;
+    static constexpr uint32_t RG = CBG * 2, GBOX = kGradW * kGradH * RG;
+    static constexpr uint32_t STAGE = GROUPS * XS + NG * GBOX;
+    static constexpr int COLS = NACC * BN;
+    static constexpr int TCOLS = COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
+    static constexpr bool TWO = TCOLS <= 256 && 3 * STAGE + 1024 <= kSmemTwo;
+    static constexpr uint32_t BUDGET = (TWO ? kSmemTwo : kSmemOne) - 1024;
+    static constexpr int STAGES = BUDGET / STAGE >= 4 ? 4 : (int)(BUDGET / STAGE);
+    static constexpr uint32_t SMEM = STAGES * STAGE + 1024;
+    static constexpr int PER_SM = TWO ? 2 : 1;
+    static_assert(CB * GROUPS * PACK == 128 && STAGES >= 2 && COLS <= 512, "tile");
+    // the last PACK - 1 pixels of the last K step lie past the box
+    static_assert(TAPS == 1 || PACK == 1 || XS >= XBOX + R, "reads past the box stay in its stage");
+};
+
+// first tap offset of accumulator a
+template <int PACK, int TAPS>
+__host__ __device__ constexpr int acc_dy(int a) { return TAPS == 1 ? 0 : PACK == 4 ? a - 1 : PACK == 2 ? a / 2 - 1 : a / 3 - 1; }
+template <int PACK, int TAPS>
+__host__ __device__ constexpr int acc_dx(int a) { return TAPS == 1 ? 0 : PACK == 4 ? -1 : PACK == 2 ? (a & 1 ? 1 : -1) : a % 3 - 1; }
+
+template <int CB, int GROUPS, int PACK, int BN, int TAPS>
+__global__ void __launch_bounds__(128, 1)
+    conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG,
+                      const GemmArgs g, int ntiles, int chunk)
+{
+    using C = WgradCfg<CB, GROUPS, PACK, BN, TAPS>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *stages = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full[C::STAGES], empty[C::STAGES], done;
+    __shared__ uint32_t tmem_sh;
+    __shared__ int fail_sh;
+    const int warp = umma::warp_index(), lane = threadIdx.x & 31;
+    const int co0 = blockIdx.y * BN, ci0 = blockIdx.z * CB * GROUPS;
+    const int k0 = blockIdx.x * chunk, nk = min(chunk, ntiles - k0);
+    const bool bias = g.db && blockIdx.z == 0;
+    const int tx = (g.W + kGradW - 1) / kGradW, ty = (g.H + kGradH - 1) / kGradH;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; s++) {
+            umma::bar_init(&full[s], 1);
+            umma::bar_init(&empty[s], bias ? 3 : 1);  // the MMAs, and the two warps that sum G
+        }
+        umma::bar_init(&done, 1);
+        umma::bar_fence_init();
+        fail_sh = 0;
+    }
+    if (warp == 0) {
+        umma::tmem_alloc(&tmem_sh, C::TCOLS);
+        umma::tmem_relinquish();
+    }
+    umma::tc_fence_before();
+    __syncthreads();
+    umma::tc_fence_after();
+    const uint32_t tmem = tmem_sh;
+
+    if (warp == 0 && lane == 0) {
+        for (int k = 0; k < nk; k++) {
+            const int s = k % C::STAGES, round = k / C::STAGES;
+            if (round > 0 && !umma::bar_wait(&empty[s], (round - 1) & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            const int tile = k0 + k, n = tile / (tx * ty), r = tile % (tx * ty);
+            const int y0 = (r / tx) * kGradH, x0 = (r % tx) * kGradW;
+            constexpr int halo = TAPS == 1 ? 0 : 1;
+            umma::bar_expect_tx(&full[s], GROUPS * C::XBOX + C::NG * C::GBOX);
+            uint8_t *st = stages + s * C::STAGE;
+#pragma unroll
+            for (int j = 0; j < GROUPS; j++)
+                umma::tma_load_4d(st + j * C::XS, &tmX, ci0 + j * CB, x0 - halo, y0 - halo, n, &full[s]);
+#pragma unroll
+            for (int j = 0; j < C::NG; j++)
+                umma::tma_load_4d(st + GROUPS * C::XS + j * C::GBOX, &tmG, co0 + j * C::CBG, x0, y0, n, &full[s]);
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = umma::make_idesc(128, BN, 1, 1);
+        for (int k = 0; k < nk; k++) {
+            const int s = k % C::STAGES, round = k / C::STAGES;
+            if (!umma::bar_wait(&full[s], round & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            umma::tc_fence_after();
+            const uint32_t x0 = umma::smem_addr(stages) + s * C::STAGE;
+            umma::Desc xd = umma::make_desc(x0, PACK > 1 ? C::R : C::XS, 8 * C::R, C::R);
+            umma::Desc gd = umma::make_desc(x0 + GROUPS * C::XS, C::GBOX, 8 * C::RG, C::RG);
+#pragma unroll 1
+            for (int r = 0; r < kGradH; r++) {
+#pragma unroll
+                for (int a = 0; a < C::NACC; a++) {
+                    constexpr int o = TAPS == 1 ? 0 : 1;
+                    const int at = (acc_dy<PACK, TAPS>(a) + o) * C::XW + acc_dx<PACK, TAPS>(a) + o;
+                    umma::mma_bf16(tmem + a * BN, xd + at * C::R, gd, idesc, (k > 0 || r > 0) ? 1u : 0u);
+                }
+                xd = xd + C::XW * C::R;
+                gd = gd + kGradW * C::RG;
+            }
+            umma::mma_commit(&empty[s]);
+        }
+        umma::mma_commit(&done);
+    } else if (warp >= 2 && bias) {
+        // thread: eight channels (chunk cc) of pixels p0, p0 + step, ...
+        constexpr int CH = BN / 8, step = 64 / CH;
+        const int cc = lane % CH, c = cc % (C::CBG / 8), p0 = (threadIdx.x - 64) / CH;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < nk; k++) {
+            const int s = k % C::STAGES, round = k / C::STAGES;
+            if (!umma::bar_wait(&full[s], round & 1)) {
+                fail_sh = 1;
+                break;
+            }
+            const uint8_t *gs = stages + s * C::STAGE + GROUPS * C::XS + (cc * 8 / C::CBG) * C::GBOX;
+#pragma unroll 4
+            for (int p = p0; p < kGradW * kGradH; p += step) {
+                // the 16-byte units of a staged pixel are swizzled by its address
+                const int u = c ^ (C::RG == 128 ? p & 7 : (p >> 1) & 3);
+                const uint4 q = *reinterpret_cast<const uint4 *>(gs + p * C::RG + 16 * u);
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    acc[2 * i] += __uint_as_float(w[i] << 16);
+                    acc[2 * i + 1] += __uint_as_float(w[i] & 0xFFFF0000u);
+                }
+            }
+            __syncwarp();
+            if (lane == 0)
+                umma::bar_arrive(&empty[s]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            for (int o = CH; o < 32; o <<= 1)
+                acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+            if (lane < CH)
+                atomicAdd(g.db + co0 + 8 * cc + e, acc[e]);
+        }
+    }
+    __syncwarp();
+
+    // accumulator rows are TMEM lanes (warp w: lanes 32w..)
+    const bool got = umma::bar_wait(&done, 0);
+    umma::tc_fence_after();
+    const int row = warp * 32 + lane;
+    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+    const int j = PACK > 1 ? row / CB : 0, ci = ci0 + (PACK > 1 ? row % CB : row);
+#pragma unroll 1
+    for (int a = 0; a < C::NACC; a++) {
+        const int dx = acc_dx<PACK, TAPS>(a) + j, tap = TAPS == 1 ? 0 : (acc_dy<PACK, TAPS>(a) + 1) * 3 + dx + 1;
+        if (dx > (TAPS == 1 ? 0 : 1))  // the same for a whole warp
+            continue;
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 16) {
+            float v[16];
+            umma::tmem_ld16(trow + a * BN + c0, v);
+            float *dst = g.dw + ((size_t)(co0 + c0) * TAPS + tap) * g.cin + ci;
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                atomicAdd(dst + (size_t)i * TAPS * g.cin, v[i]);
+        }
+    }
+    if (threadIdx.x == 0 && (!got || fail_sh) && g.status)
+        atomicExch(g.status, 1);
+    umma::tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        umma::tmem_dealloc(tmem, C::TCOLS);
 }
 
 // ------------------------------------------------------------------ host
@@ -493,27 +714,27 @@ bool map_matrix(CUtensorMap *m, const void *base, int cols, int rows, int cb, in
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MODE, int CBA, int CBB, int BN>
-bool launch(const CUtensorMap &ta, const CUtensorMap &tb, const GemmArgs &g, dim3 grid, cudaStream_t s)
-{
-    using C = GemmCfg<MODE, CBA, CBB, BN>;
-    auto k = conv_gemm_kernel<MODE, CBA, CBB, BN>;
-    static bool configured = false;
-    if (!configured) {
-        if (!FMVD_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM)))
-            return false;
-        configured = true;
-    }
-    k<<<grid, 128, C::SMEM, s>>>(ta, tb, g);
-    rl_count_launch(1);
-    return FMVD_CHECK(cudaGetLastError());
-}
-
 // pixel box of 'count' pixels on a W-wide image
 void pixel_box(int W, int count, int &bw, int &bh)
 {
     bw = W < count ? W : count;
     bh = count / bw;
+}
+
+// Opts a kernel in to its dynamic shared memory (once per process; the
+// devices of a process are alike) and reads the multiprocessor count.
+template <typename K>
+bool configure(K kern, uint32_t smem, int &sms)
+{
+    if (sms)
+        return true;
+    int dev = 0, n = 0;
+    if (!FMVD_CHECK(cudaGetDevice(&dev)) ||
+        !FMVD_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) ||
+        !FMVD_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
+        return false;
+    sms = n;
+    return true;
 }
 
 template <int CB, int BN>
@@ -523,15 +744,8 @@ bool launch_persistent(const CUtensorMap &ta, const CUtensorMap &tb, const GemmA
     using C = PersistCfg<CB, BN>;
     auto k = conv_gemm_persistent<CB, BN>;
     static int sms = 0;
-    static bool configured = false;
-    if (!configured) {
-        int dev = 0;
-        if (!FMVD_CHECK(cudaGetDevice(&dev)) ||
-            !FMVD_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
-            !FMVD_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM)))
-            return false;
-        configured = true;
-    }
+    if (!configure(k, C::SMEM, sms))
+        return false;
     // CTAs per SM: tensor memory (512 columns) and shared memory allow
     const int by_tmem = 512 / C::TCOLS;
     const int by_smem = (int)(200u * 1024u / C::SMEM);
@@ -559,16 +773,64 @@ bool dispatch_persistent(int bn, const CUtensorMap &ta, const CUtensorMap &tb, c
     }
 }
 
-template <int MODE, int CBA, int CBB>
-bool dispatch_bn(int bn, const CUtensorMap &ta, const CUtensorMap &tb, const GemmArgs &g, dim3 grid, cudaStream_t s)
+bool aligned32(const void *p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; }
+
+template <int CB, int NB, int BN>
+bool launch_halo(const CUtensorMap &ta, const CUtensorMap &tb, const GemmArgs &g, cudaStream_t s)
 {
-    switch (bn) {
-#define X(B) \
-    case B: return launch<MODE, CBA, CBB, B>(ta, tb, g, grid, s);
-        FMVD_BN_CASES(X)
+    using C = HaloCfg<CB, NB, BN>;
+    auto k = conv_halo<CB, NB, BN>;
+    static int sms = 0;
+    if (!configure(k, C::SMEM, sms))
+        return false;
+    const int ntiles = g.N * ((g.H + kTileH - 1) / kTileH) * (g.W / kTileW);
+    // CTAs per SM: tensor memory (512 columns), shared memory (228 KB, 1 KB of
+    // it per CTA reserved), registers
+    int per_sm = (int)(228u * 1024u / (C::SMEM + 1024u));
+    per_sm = std::max(1, std::min(per_sm, std::min(512 / C::TCOLS, 3)));
+    k<<<std::min(ntiles, sms * per_sm), kPersistentThreads, C::SMEM, s>>>(ta, tb, g, ntiles);
+    rl_count_launch(1);
+    return FMVD_CHECK(cudaGetLastError());
+}
+
+// The halo kernel for this layer, or null where its weights do not fit.
+using HaloLaunch = bool (*)(const CUtensorMap &, const CUtensorMap &, const GemmArgs &, cudaStream_t);
+HaloLaunch halo_for(int cin, int cout)
+{
+    switch (cin * 1024 + cout) {
+#define X(CI, CB, NB, BN) \
+    case CI * 1024 + BN: return launch_halo<CB, NB, BN>;
+        X(32, 32, 1, 16) X(32, 32, 1, 32) X(32, 32, 1, 64) X(32, 32, 1, 128)
+        X(64, 64, 1, 16) X(64, 64, 1, 32) X(64, 64, 1, 64) X(64, 64, 1, 128)
+        X(128, 64, 2, 32) X(128, 64, 2, 64)
 #undef X
-    default: report_error("fmvd: unsupported GEMM N tile"); return false;
+    default: return nullptr;
     }
+}
+
+template <int CB, int GROUPS, int PACK, int BN, int TAPS>
+bool launch_wgrad(const CUtensorMap &tx, const CUtensorMap &tg, const GemmArgs &g, cudaStream_t s)
+{
+    using C = WgradCfg<CB, GROUPS, PACK, BN, TAPS>;
+    auto k = conv_wgrad_kernel<CB, GROUPS, PACK, BN, TAPS>;
+    static int sms = 0;
+    if (!configure(k, C::SMEM, sms))
+        return false;
+    const int ntiles = g.N * ((g.H + kGradH - 1) / kGradH) * ((g.W + kGradW - 1) / kGradW);
+    // pixels per CTA: a bounded accumulation (see the kernel), at least 8 tiles
+    const long long parts = (long long)g.taps * ((g.cout + 127) / 128) * ((g.cin + 255) / 256);
+    const int chunk = (int)std::min<long long>(ntiles, std::max<long long>(8, (ntiles * parts + 1183) / 1184));
+    const dim3 grid((ntiles + chunk - 1) / chunk, g.cout / BN, g.cin / (CB * GROUPS));
+    k<<<grid, 128, C::SMEM, s>>>(tx, tg, g, ntiles, chunk);
+    rl_count_launch(1);
+    return FMVD_CHECK(cudaGetLastError());
+}
+
+template <int CB, int GROUPS, int PACK, int BN>
+bool wgrad_taps(const CUtensorMap &tx, const CUtensorMap &tg, const GemmArgs &g, cudaStream_t s)
+{
+    return g.taps == 9 ? launch_wgrad<CB, GROUPS, PACK, BN, 9>(tx, tg, g, s)
+                       : launch_wgrad<CB, GROUPS, PACK, BN, 1>(tx, tg, g, s);
 }
 
 } // namespace
@@ -589,8 +851,9 @@ bool conv_forward(const ConvDesc &c, cudaStream_t s)
     }
     int bw, bh;
     pixel_box(c.W, 128, bw, bh);
+    const HaloLaunch halo = c.taps == 9 ? halo_for(c.cin, c.cout) : nullptr;
     CUtensorMap ta, tb;
-    if (!map_nhwc(&ta, c.in, c.cin, c.W, c.H, c.N, cb, bw, bh) ||
+    if (!map_nhwc(&ta, c.in, c.cin, c.W, c.H, c.N, cb, halo ? kBoxW : bw, halo ? kBoxH : bh) ||
         !map_matrix(&tb, c.weight, c.taps * c.cin, c.cout, cb, bn)) {
         report_error("fmvd: tensor map encoding failed");
         return false;
@@ -616,14 +879,14 @@ bool conv_forward(const ConvDesc &c, cudaStream_t s)
     g.mask_ld = c.mask_ld ? c.mask_ld : c.cout;
     g.relu = c.relu;
     g.status = c.status;
+    // 32-byte accesses in the epilogue where sixteen channels of every tensor
+    // start on a 32-byte boundary (the channel counts are multiples of 16)
+    g.vec = aligned32(c.bias) && aligned32(c.add) && aligned32(c.mask) && aligned32(c.out) &&
+            (g.add_ld | g.mask_ld | g.out_ld | g.out_coff) % 16 == 0;
+    if (halo)
+        return halo(ta, tb, g, s);
     const int ntiles_n = c.cout / bn;
     const int ntiles = c.N * (c.H / bh) * (c.W / bw) * ntiles_n;
-    if (cb == 32 && bn <= 32) {
-        // 32-channel operands with a narrow N: one CTA per tile keeps more
-        // K blocks in flight per SM (measured faster on B200)
-        const dim3 grid((unsigned)(ntiles / ntiles_n), (unsigned)ntiles_n, 1);
-        return dispatch_bn<0, 32, 32>(bn, ta, tb, g, grid, s);
-    }
     return cb == 64 ? dispatch_persistent<64>(bn, ta, tb, g, ntiles, ntiles_n, s)
                     : dispatch_persistent<32>(bn, ta, tb, g, ntiles, ntiles_n, s);
 }
@@ -638,46 +901,37 @@ bool conv_wgrad(const WgradDesc &c, cudaStream_t s)
     const int cba = c.cout >= 64 ? 64 : 32;
     const int cbb = c.cin >= 64 ? 64 : 32;
     const int bn = c.cin > 256 ? 256 : c.cin;
-    const long long pixels = (long long)c.N * c.H * c.W;
-    if (c.cout % cba || c.cin % cbb || c.cin % bn || bn % 16 || (c.taps != 1 && c.taps != 9) ||
-        (c.H * c.W) % kKP || (c.W < kKP ? kKP % c.W : c.W % kKP)) {
+    if (c.cout % cba || c.cin % cbb || c.cin % bn || (bn != 32 && bn != 64 && bn != 128 && bn != 256) ||
+        (c.taps != 1 && c.taps != 9) || (c.H * c.W) % 64 || (c.W < 64 ? 64 % c.W : c.W % 64)) {
         report_error("fmvd: unsupported weight-gradient geometry");
         return false;
     }
-    int bw, bh;
-    pixel_box(c.W, kKP, bw, bh);
-    CUtensorMap ta, tb;
-    if (!map_nhwc(&ta, c.grad, c.cout, c.W, c.H, c.N, cba, bw, bh) ||
-        !map_nhwc(&tb, c.in, c.cin, c.W, c.H, c.N, cbb, bw, bh)) {
+    // N tile (output channels): what tensor memory holds beside every tap
+    const int nt = c.cin >= 128 ? 32 : c.cin == 64 ? (cba == 64 ? 64 : 32)
+                                                   : (c.cout % 128 == 0 ? 128 : cba == 64 ? 64 : 32);
+    const int halo = c.taps == 9 ? 2 : 0;
+    CUtensorMap tx, tg;
+    if (!map_nhwc(&tx, c.in, c.cin, c.W, c.H, c.N, cbb, kGradW + halo, kGradH + halo) ||
+        !map_nhwc(&tg, c.grad, c.cout, c.W, c.H, c.N, nt >= 64 ? 64 : 32, kGradW, kGradH)) {
         report_error("fmvd: tensor map encoding failed");
         return false;
     }
-    const int total = (int)(pixels / kKP);
-    const int co_tiles = (c.cout + 127) / 128;
-    const int ci_tiles = c.cin / bn;
-    // split K so that the grid covers the GPU a few times over
-    const long long base = (long long)c.taps * co_tiles * ci_tiles;
-    int kchunk = (int)((total * base + 1183) / 1184);
-    if (kchunk < 16)
-        kchunk = 16;
-    if (kchunk > total)
-        kchunk = total;
     GemmArgs g{};
     g.N = c.N;
     g.H = c.H;
     g.W = c.W;
-    g.bw = bw;
-    g.bh = bh;
     g.taps = c.taps;
     g.cin = c.cin;
     g.cout = c.cout;
-    g.kchunk = kchunk;
     g.dw = c.dw;
+    g.db = c.db;
     g.status = c.status;
-    const dim3 grid((unsigned)(c.taps * co_tiles), (unsigned)((total + kchunk - 1) / kchunk), (unsigned)ci_tiles);
-    if (cba == 64)
-        return cbb == 64 ? dispatch_bn<1, 64, 64>(bn, ta, tb, g, grid, s) : dispatch_bn<1, 64, 32>(bn, ta, tb, g, grid, s);
-    return cbb == 64 ? dispatch_bn<1, 32, 64>(bn, ta, tb, g, grid, s) : dispatch_bn<1, 32, 32>(bn, ta, tb, g, grid, s);
+    if (c.cin >= 128)
+        return wgrad_taps<64, 2, 1, 32>(tx, tg, g, s);
+    if (c.cin == 64)
+        return nt == 64 ? wgrad_taps<64, 1, 2, 64>(tx, tg, g, s) : wgrad_taps<64, 1, 2, 32>(tx, tg, g, s);
+    return nt == 128 ? wgrad_taps<32, 1, 4, 128>(tx, tg, g, s)
+                     : nt == 64 ? wgrad_taps<32, 1, 4, 64>(tx, tg, g, s) : wgrad_taps<32, 1, 4, 32>(tx, tg, g, s);
 }
 
 } // namespace unet

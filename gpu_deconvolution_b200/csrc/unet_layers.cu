@@ -1,7 +1,7 @@
 // Element-wise and reduction kernels of the warm-start network (BF16 NHWC
 // activations, FP32 arithmetic): input normalisation and 3x3 patch
 // extraction of the first layer, 2x2 average pooling / nearest upsampling
-// and their gradients, bias gradients, the 1x1 output layer with the L1 loss,
+// and their gradients, the 1x1 output layer with the L1 loss,
 // and the Adam update that also writes the bf16 weights of the forward and
 // data-gradient GEMMs.
 #include "fmvd_internal.h"
@@ -255,35 +255,6 @@ __global__ void upsample_grad_kernel(const bf16 *g_up, const bf16 *act, bf16 *g,
     }
 }
 
-// db[c] += sum over pixels of g[p][c]: thread (row r, chunk cc) sums 8
-// channels over pixels r, r + rows, ...; block partials through shared memory.
-__global__ void bias_grad_kernel(const bf16 *g, size_t P, int C, float *db)
-{
-    __shared__ float sdb[256];
-    const int C8 = C / 8;
-    const int rows = blockDim.x / C8;
-    const int cc = threadIdx.x % C8, r = threadIdx.x / C8;
-    for (int i = threadIdx.x; i < C; i += blockDim.x)
-        sdb[i] = 0.f;
-    __syncthreads();
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (r < rows) {
-        for (size_t p = blockIdx.x * (size_t)rows + r; p < P; p += (size_t)gridDim.x * rows) {
-            float v[8];
-            load8(g + p * C + 8 * cc, v);
-#pragma unroll
-            for (int e = 0; e < 8; e++)
-                acc[e] += v[e];
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e++)
-            atomicAdd(&sdb[8 * cc + e], acc[e]);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < C; i += blockDim.x)
-        atomicAdd(db + i, sdb[i]);
-}
-
 // y[p] = sum_c act[p][c] w[c] + b (normalised units); optional outputs:
 // the estimate y * s[n], and with a target the L1 loss and its gradient.
 __global__ void output_kernel(const bf16 *act, const float *w, const float *b, int C, int N, int HW,
@@ -484,16 +455,6 @@ bool pool_grad(const bf16 *g_pool, const bf16 *g_skip, const bf16 *act, bf16 *g,
 bool upsample_grad(const bf16 *g_up, const bf16 *act, bf16 *g, int N, int H, int W, int C, cudaStream_t s)
 {
     upsample_grad_kernel<<<grid_for((size_t)N * H * W * C / 8), 256, 0, s>>>(g_up, act, g, N, H, W, C);
-    rl_count_launch(1);
-    return FMVD_CHECK(cudaGetLastError());
-}
-
-bool bias_grad(const bf16 *g, size_t P, int C, float *db, cudaStream_t s)
-{
-    // 256 threads: C / 8 channel chunks by 256 / (C / 8) pixel rows
-    const size_t rows = 256 / (C / 8);
-    const size_t need = (P + rows - 1) / rows;
-    bias_grad_kernel<<<(int)(need < 148 * 8 ? need : 148 * 8), 256, 0, s>>>(g, P, C, db);
     rl_count_launch(1);
     return FMVD_CHECK(cudaGetLastError());
 }

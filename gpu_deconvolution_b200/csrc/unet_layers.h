@@ -25,7 +25,6 @@ bool pool_grad(const __nv_bfloat16 *g_pool, const __nv_bfloat16 *g_skip, const _
                int N, int H, int W, int C, cudaStream_t s);
 bool upsample_grad(const __nv_bfloat16 *g_up, const __nv_bfloat16 *act, __nv_bfloat16 *g, int N, int H, int W, int C,
                    cudaStream_t s);
-bool bias_grad(const __nv_bfloat16 *g, size_t P, int C, float *db, cudaStream_t s);
 bool output_layer(const __nv_bfloat16 *act, const float *w, const float *b, int C, int N, int HW, const float *scale,
                   float *estimate, const float *target, float *gy, float *loss, cudaStream_t s);
 bool output_grad(const __nv_bfloat16 *act, const float *w, int C, size_t P, const float *gy, __nv_bfloat16 *g_act,

@@ -132,8 +132,9 @@ bool wgrad(const Net &n, const Layer &l, const bf16 *g_out, const bf16 *in, int 
     c.cout = l.cout;
     c.taps = l.taps;
     c.dw = n.grads + l.w_off;
+    c.db = n.grads + l.b_off;
     c.status = n.status;
-    return conv_wgrad(c, s) && bias_grad(g_out, (size_t)N * c.H * c.W, l.cout, n.grads + l.b_off, s);
+    return conv_wgrad(c, s);
 }
 
 bool refresh_weights(Net &n, cudaStream_t s)
