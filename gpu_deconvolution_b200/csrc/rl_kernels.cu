@@ -40,7 +40,16 @@ static unsigned long long g_launches = 0;
 unsigned long long rl_launch_count() { return g_launches; }
 void rl_count_launch(unsigned long long n) { g_launches += n; }
 
-// Work planes are row-major: element (y, x) of pair p at C[(p * H + y) * W + x].
+// Work planes are row-major, element (y, x) of pair p at
+// C[(p * H + y) * W + x], but for planes of 1024 rows: there x is exchanged
+// within its column block for x ^ f(y), f the bank swizzle of the column
+// pass's tile.  That costs the row passes nothing (f is fixed per row, so a
+// lane's elements stay T apart), and the column pass fills its tile with
+// 16-byte copies that need no swizzle of their own.
+struct RowSwizzle {
+    int shift, mask;  // f(y) = (y >> shift) & mask; mask 0: none
+    __device__ __forceinline__ int f(int y) const { return (y >> shift) & mask; }
+};
 
 __device__ __forceinline__ int clamp_src(int i, int n, int border)
 {
@@ -100,6 +109,7 @@ struct RowArgs {
     int last;
     int bulk_data;      // data rows may be fetched with 16-byte bulk copies
     int group_floats;   // warp engine: shared floats per group (transpose + prefetch)
+    RowSwizzle sw;      // storage order of the work planes' rows
     const float2 *twN;  // lines above 1024: exp(-2 pi i n / W), n < W
 };
 
@@ -269,7 +279,10 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
     const bool valid = yr < H;
     const int y = valid ? yr : H - 1;
     const int p = blockIdx.y;
+    // element x = t + T m; the swizzle is below 8, so lanes stay among the T
+    // of one m, but for T = 4 its upper bit picks the neighbouring m
     float2 *row = a.b.C + ((size_t)p * H + y) * W;
+    const int sw = a.sw.f(y), tsw = t ^ (sw & (T - 1)), msw = T < 8 ? sw / T : 0;
     RowWork<MODE, BITS, NOOUT, SMEM> work(a, p, y);
 
     // Rows the element-wise step needs are fetched by the bulk-copy engine
@@ -338,7 +351,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
         if (pass == 0) {
 #pragma unroll
             for (int m = 0; m < E; m++) {
-                const float2 x = row[t + T * m];
+                const float2 x = row[tsw + T * (T < 8 ? m ^ msw : m)];
                 v[m] = make_float2(x.x, -x.y);
             }
         }
@@ -389,7 +402,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, FMVD_ROW_MIN_BLOCKS) row_pass_
     if (valid) {
 #pragma unroll
         for (int m = 0; m < E; m++)
-            row[t + T * m] = v[m];
+            row[tsw + T * (T < 8 ? m ^ msw : m)] = v[m];
     }
 }
 
@@ -448,11 +461,14 @@ __device__ __forceinline__ float2 lds2(uint32_t addr)
 // 128-byte wavefront) at a time, and f spreads every access of a transform
 // over the sixteen slots of that wavefront:
 //   T = 32: sixteen lanes hold sixteen consecutive rows of one column, so f
-//     steps by one slot per 128 bytes of rows;
+//     steps by one slot per 128 bytes of rows.  It separates column pairs, so
+//     the work plane itself is stored in this order (RowSwizzle);
 //   T < 32: sixteen lanes hold eight (T = 4: four) rows of two (four)
 //     neighbouring columns, so f steps by two (four) slots and a column pair
-//     stays one aligned 16-byte unit: the tile is filled and written back 16
-//     bytes at a time.
+//     stays one aligned 16-byte unit.
+// Either way the tile is filled and written back 16 bytes at a time (8-byte
+// copies take a shared-memory cycle per row they touch: 0.75 M conflicts per
+// launch of three 1024 x 1024 pairs).
 // With T = 16 the two lines of a warp are interleaved lane by lane (line =
 // lane & 1) to get eight rows of two columns in a half-warp.
 // f uses the low bits of y only, so that for u, k < T it is linear in XOR:
@@ -478,8 +494,8 @@ struct ColTile {
 };
 
 // H-point transform of one tile column (the WarpFft<H> four-step): wbase =
-// tile | Q(t) (transpose writes, element k1 at row T k1 + (t ^ k1 mod T)),
-// rbase = (tile + 8 FC T t) | Q(t) (reads of row-block t).
+// tile + Q(t) (transpose writes, element k1 at row T k1 + (t ^ k1 mod T)),
+// rbase = wbase + 8 FC T t (reads of row-block t).
 template <int H, int FC, int DIR>
 __device__ __forceinline__ void col_fft(float2 *v, const float2 *__restrict__ tw, uint32_t wbase, uint32_t rbase, int t)
 {
@@ -508,11 +524,6 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-
 // Column pass for H <= 1024: CW warps per block, G = 32 / T columns per
 // warp, FC = CW * G columns per block.  The FC-column tile is filled by
 // cp.async (whole rows of the tile, 16 to 128 bytes, coalesced), each group
@@ -546,30 +557,27 @@ __global__ void __launch_bounds__(CW * 32, FMVD_COL_MIN_BLOCKS * (8 / CW)) col_p
 
     const uint32_t s0 = smem_u32addr(smem);
     const uint32_t base = (s0 + TL::align - 1) & ~(TL::align - 1);
-    // fill: U-byte units; a thread keeps its unit of the row and steps RI
-    // rows at a time, a multiple of the rows f tells apart, so its swizzle
-    // is a constant
-    constexpr int U = TL::pairs ? 16 : 8, UR = TL::RB / U, RI = NT / UR;
+    // fill in 16-byte units (a column pair): a thread keeps its unit of the
+    // row and steps RI rows at a time, a multiple of the rows f tells apart,
+    // so its swizzle is a constant (none with T = 32, where the plane is
+    // stored swizzled)
+    constexpr int PR = TL::RB / 16, RI = NT / PR;
     static_assert(RI % TL::rows == 0 && H % RI == 0, "a thread's rows share one swizzle");
     {
-        const int y = threadIdx.x / UR, u = threadIdx.x % UR;
-        const uint32_t dst = base + TL::RB * y + ((uint32_t)(U * u) ^ (8u * TL::f(y)));
-        const char *src = reinterpret_cast<const char *>(C + (size_t)y * W) + U * u;
+        const int y = threadIdx.x / PR, u = threadIdx.x % PR;
+        const uint32_t dst = base + TL::RB * y + (TL::pairs ? (16u * u) ^ (8u * TL::f(y)) : 16u * u);
+        const char *src = reinterpret_cast<const char *>(C + (size_t)y * W) + 16 * u;
         const size_t pitch = (size_t)RI * W * sizeof(float2);
 #pragma unroll 8
-        for (int i = 0; i < H / RI; i++) {
-            if constexpr (TL::pairs)
-                cp_async16(dst + RI * TL::RB * i, src + pitch * i);
-            else
-                cp_async8(dst + RI * TL::RB * i, src + pitch * i);
-        }
+        for (int i = 0; i < H / RI; i++)
+            cp_async16(dst + RI * TL::RB * i, src + pitch * i);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     const int t = TL::pos(lane), c = warp * G + TL::line(lane);
     const uint32_t q = TL::RB * t + 8u * (c ^ TL::f(t));
-    uint32_t wbase = base | q, rbase = (base + TL::align * t) | q;
+    uint32_t wbase = base + q, rbase = wbase + TL::align * t;
     const float2 *tw = a.tw;
     float2 v[E];
 #pragma unroll
@@ -600,18 +608,10 @@ __global__ void __launch_bounds__(CW * 32, FMVD_COL_MIN_BLOCKS * (8 / CW)) col_p
     for (int m = 0; m < E; m++)
         sts2(wbase + TL::align * m, make_float2(v[m].x, -v[m].y));
     __syncthreads();
-    constexpr int PR = TL::RB / 16;
 #pragma unroll 4
     for (int n = threadIdx.x; n < H * PR; n += NT) {
         const int y = n / PR, u = n % PR;
-        const uint32_t row = base + TL::RB * y;
-        float4 e;
-        if constexpr (TL::pairs) {
-            e = lds4(row + ((16u * u) ^ (8u * TL::f(y))));
-        } else {
-            const float2 e0 = lds2(row + ((16u * u) ^ (8u * TL::f(y)))), e1 = lds2(row + ((16u * u + 8) ^ (8u * TL::f(y))));
-            e = make_float4(e0.x, e0.y, e1.x, e1.y);
-        }
+        const float4 e = lds4(base + TL::RB * y + (TL::pairs ? (16u * u) ^ (8u * TL::f(y)) : 16u * u));
         *reinterpret_cast<float4 *>(C + (size_t)y * W + 2 * u) = e;
     }
 }
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
     float2 *const buf = lbuf + (size_t)r * PF2;
     const int y = blockIdx.x * 2 + h;
     const int p = blockIdx.y;
-    float2 *row = a.b.C + ((size_t)p * a.d.H + y) * N + r * kLineM;
+    float2 *row = a.b.C + ((size_t)p * a.d.H + y) * N + r * kLineM + (t ^ a.sw.f(y));  // element t + 16 m at row[16 m]
     RowWork<MODE, BITS, NOOUT, SMEM, false> work(a, p, y);
 
     // operand rows staged by bulk copies, issued now by one thread per row
@@ -759,7 +759,7 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
     } else {
 #pragma unroll
         for (int m = 0; m < E; m++) {
-            const float2 x = row[t + T * m];
+            const float2 x = row[T * m];
             v[m] = make_float2(x.x, -x.y);
         }
     }
@@ -808,101 +808,117 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
     }
 #pragma unroll
     for (int m = 0; m < E; m++)
-        row[t + T * m] = v[m];
+        row[T * m] = v[m];
 }
 
-// Column tile of the line engine: two columns, element (y, c) at float2
-// 2 y + (c ^ ((y >> 3) & 1)): sixteen consecutive rows of one column fall in
-// sixteen distinct 8-byte slots of a 256-byte window.  With the tile on a
-// 256-byte boundary, row y = 512 r + 16 a + u (u < 16) of column c is at
-// byte 8192 r + 256 a + 8 Q_c(u), Q_c(u) = 2 u + (c ^ ((u >> 3) & 1)), and
-// Q_c is XOR-linear: Q_c(t ^ k) = Q_c(t) ^ R16(k), R16(k) = 2 k + ((k >> 3) & 1).
-__device__ __forceinline__ int coltile_r(int y, int c) { return 2 * y + (c ^ ((y >> 3) & 1)); }
-__host__ __device__ constexpr uint32_t coltile16_r(int k) { return 2u * k + ((k >> 3) & 1); }
+// Column tile of the line engine: four columns, row y at byte 32 y, element
+// (y, c) in slot c ^ f(y), f(y) = 2 ((y >> 2) & 1).  Lane l of a warp holds
+// column l & 1 of the warp's pair at position l >> 1, so sixteen lanes hold
+// eight rows of two columns, and f puts them in sixteen distinct slots of a
+// wavefront.  Column pairs stay together (16-byte fill and write-back).  Row
+// y = 512 r + 16 a + (t ^ k) (t, k < 16) is at byte
+// 16384 r + 512 a + (Q(t) ^ R(k)), Q(t) = 32 t + 8 (c ^ f(t)),
+// R(k) = 32 k + 8 f(k).
+struct LineTile {
+    static constexpr int RB = 32;
+    static __host__ __device__ constexpr uint32_t f(int y) { return 2u * ((y >> 2) & 1); }
+    static __host__ __device__ constexpr uint32_t R(int k) { return (uint32_t)RB * k + 8u * f(k); }
+};
 
 // 512-point transform (WarpFft<512>: T = 16, E = 32) of one sub-line of a
-// line-engine column tile, its own rows as transpose space:
-// wbase = sub-line start | 8 Q_c(t), rbase = (sub-line start + 256 t) | 8 Q_c(t).
+// line-engine column tile, its own rows as transpose space: wbase = sub-line
+// start + Q(t), rbase = wbase + 512 t.
 template <int DIR, typename TW>
 __device__ __forceinline__ void col_fft_512(float2 *v, const TW &tw, uint32_t wbase, uint32_t rbase, int t)
 {
     using WF = WarpFft<kLineM>;
+    using TL = LineTile;
     Dft<32, DIR>::run(v);
     WF::template twiddle<DIR>(v, tw, t);
 #pragma unroll
     for (int k1 = 0; k1 < 32; k1++)
-        sts2((wbase ^ (8u * coltile16_r(k1 & 15))) + 256u * k1, v[k1]);
+        sts2((wbase ^ TL::R(k1 & 15)) + 16u * TL::RB * k1, v[k1]);
     __syncwarp();
 #pragma unroll
     for (int s = 0; s < 2; s++)
 #pragma unroll
         for (int j = 0; j < 16; j++)
-            v[s * 16 + j] = lds2((rbase ^ (8u * coltile16_r(j))) + 4096u * s);
+            v[s * 16 + j] = lds2((rbase ^ TL::R(j)) + 256u * TL::RB * s);
     __syncwarp();
     Dft<16, DIR>::run(v);
     Dft<16, DIR>::run(v + 16);
     WF::reorder(v);
 }
 
-// Column pass for H = R * 512: R warps, two columns per block (half-warp cc
-// of warp r is group r of column cc).  Spectrum in launch layout: block bx,
-// register m, thread tid at spec[(bx * 32 + m) * (32 R) + tid].  Resident
-// blocks per SM: 16 / R, except 4 (not 5) for R = 3, where the register cap of
-// five blocks spills and four run 2 % faster.
+// Column pass for H = R * 512: R warps per column pair (lane l of the warp
+// (r, pair) is in group r of column 2 pair + (l & 1)), four columns per block,
+// so that a row of the tile is a whole 32-byte sector and comes by 16-byte
+// copies.  With two columns per block, filled eight bytes at a time, a launch
+// of one 2560 x 2560 pair took 79 us and 510 MB of L2 traffic, now 66 us and
+// 370 MB (1536 x 1536: 32 -> 24 us);
+// ten iterations of 1400 x 1400 x 12 went from 17.7 to 14.4 ms.  Against two
+// columns filled by 16-byte copies: 13 % faster at R = 3, 9 % at 4, 11 % at 5,
+// 3 % at 6, 5 % at 8, 0.6 % slower at 7.  Bound by its two block barriers per
+// radix-R step, issue and L2 latency.
+// Spectrum in launch layout: warp w = pair * R + r of the plane, register m,
+// lane l at spec[(w * 32 + m) * 32 + l].
+constexpr int kLineColumns = 4;
+// Resident blocks per SM
 template <int R>
-constexpr int col_r_blocks() { return R == 3 ? 4 : 16 / R; }
+__host__ __device__ constexpr int col_r_blocks() { return R == 3 ? 3 : R <= 5 ? 2 : 1; }
 
 template <int R, bool DSTEP>
-__global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const ColArgs a)
+__global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_pass_r(const ColArgs a)
 {
     using WF = WarpFft<kLineM>;
     static_assert(WF::T == 16 && WF::E == 32, "sub-lines are 512-point half-warp transforms");
-    constexpr int E = WF::E, H = R * kLineM, NT = R * 32;
+    constexpr int E = WF::E, H = R * kLineM, FC = kLineColumns, PAIRS = FC / 2, NT = R * 32 * PAIRS;
+    using TL = LineTile;
+    constexpr uint32_t RB = TL::RB;
     extern __shared__ __align__(16) float smem[];
     const uint32_t s0 = smem_u32addr(smem);
-    const uint32_t base = (s0 + 255u) & ~255u;
-    float2 *tile = reinterpret_cast<float2 *>(reinterpret_cast<char *>(smem) + (base - s0));
+    const uint32_t base = (s0 + 511u) & ~511u;
     const int W = a.W;
     const int p = blockIdx.y;
-    float2 *C = a.C + (size_t)p * H * W + 2 * blockIdx.x;
+    float2 *C = a.C + (size_t)p * H * W + FC * blockIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int pair = (threadIdx.x >> 5) / R, r = (threadIdx.x >> 5) % R;
+    const float2 *sp = a.spec + (size_t)(blockIdx.x * (PAIRS * R) + (threadIdx.x >> 5)) * (E * 32) + lane;
     // this block's slice of the spectrum (contiguous in the launch layout)
     // is brought into L2 while the tile loads and the first transform runs
     pdl_launch_dependents();
     if (threadIdx.x == 0)
-        bulk_prefetch_l2(a.spec + (size_t)blockIdx.x * E * NT, (uint32_t)(E * NT * sizeof(float2)));
+        bulk_prefetch_l2(sp, (uint32_t)(E * NT * sizeof(float2)));
     pdl_wait();
 #pragma unroll 8
-    for (int i = 0; i < 2 * H / NT; i++) {
-        const int u = threadIdx.x + i * NT;
-        const int y = u >> 1, c = u & 1;
-        cp_async8(base + 8 * coltile_r(y, c), C + (size_t)y * W + c);
+    for (int n = threadIdx.x; n < H * PAIRS; n += NT) {
+        const int y = n / PAIRS, u = n % PAIRS;
+        cp_async16(base + RB * y + ((16u * u) ^ (8u * TL::f(y))), C + (size_t)y * W + 2 * u);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int r = threadIdx.x >> 5;
-    const int cc = (threadIdx.x >> 4) & 1;
-    const int t = threadIdx.x & 15;
-    const uint32_t q = 8u * (2 * t + (cc ^ ((t >> 3) & 1)));
-    const uint32_t col = base + q;                  // + 8192 j + 256 m: row 512 j + t + 16 m
-    const uint32_t seg = base + 8192u * r;          // this group's sub-line
-    const uint32_t wbase = seg | q, rbase = (seg + 256u * t) | q;
+    const int t = lane >> 1;
+    const uint32_t q = RB * t + 8u * ((2 * pair + (lane & 1)) ^ TL::f(t));
+    const uint32_t col = base + q;                  // + 512 RB j + 16 RB m: row 512 j + t + 16 m
+    const uint32_t seg = base + 512u * RB * r;      // this group's sub-line
+    const uint32_t wbase = seg + q, rbase = wbase + 16u * RB * t;
 
-    // The radix-R step of both columns in place in the tile: each half-warp
+    // The radix-R step of every column in place in the tile: each half-warp
     // takes blocks of 16 positions n1 of its column (block b = r, r + R, ...)
     // and runs the R-point DFT over the rows 512 q + n1 (q < R); with CONJ the
     // results are stored conjugated.  The tile address of row 512 q + 16 b + t
-    // of this column is col + 8192 q + 256 b.
+    // of this column is col + 512 RB q + 16 RB b.
     const auto column_dft = [&](auto conj_out) {
 #pragma unroll 1
         for (int b = r; b < kLineM / 16; b += R) {
             float2 z[R];
 #pragma unroll
             for (int q = 0; q < R; q++)
-                z[q] = lds2(col + 8192u * q + 256u * b);
+                z[q] = lds2(col + 512u * RB * q + 16u * RB * b);
             SmallDft<R>::run(z);
 #pragma unroll
             for (int q = 0; q < R; q++)
-                sts2(col + 8192u * q + 256u * b, decltype(conj_out)::value ? make_float2(z[q].x, -z[q].y) : z[q]);
+                sts2(col + 512u * RB * q + 16u * RB * b, decltype(conj_out)::value ? make_float2(z[q].x, -z[q].y) : z[q]);
         }
     };
 
@@ -910,7 +926,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
     const auto column_sum = [&](float2 *v) {
 #pragma unroll
         for (int m = 0; m < E; m++)
-            v[m] = lds2(col + 256u * m);
+            v[m] = lds2(col + 16u * RB * m);
 #pragma unroll
         for (int j = 1; j < R; j++) {
             const float2 cj = line_coefficient<R>(a.twN, r, j);
@@ -919,7 +935,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
                 asm volatile("" ::: "memory");  // bounds the loads in flight
 #pragma unroll
                 for (int m = m0; m < m0 + 8; m++)
-                    v[m] = cadd(v[m], cmul(lds2(col + 8192u * j + 256u * m), cj));
+                    v[m] = cadd(v[m], cmul(lds2(col + 512u * RB * j + 16u * RB * m), cj));
             }
         }
         asm volatile("" ::: "memory");
@@ -930,7 +946,6 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
     // the same forward pipeline then runs frequency -> space.  The rolled
     // loop keeps one copy of the transform (its table loads are not kept
     // live from one copy to the next).
-    const float2 *sp = a.spec + (size_t)blockIdx.x * E * NT + threadIdx.x;
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 0) {
@@ -939,7 +954,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
                 __syncthreads();  // every block of positions has its radix-R step
 #pragma unroll
                 for (int m = 0; m < E; m++)
-                    v[m] = lds2(col + 8192u * r + 256u * m);  // row 512 r + t + 16 m: this group's sub-line
+                    v[m] = lds2(wbase + 16u * RB * m);  // row 512 r + t + 16 m: this group's sub-line
                 __syncwarp();  // read before this warp's transposes overwrite its segment
             } else {
                 column_sum(v);
@@ -955,7 +970,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
             asm volatile("" ::: "memory");
 #pragma unroll
             for (int m = m0; m < m0 + 8; m++) {
-                const float2 z = cmul(v[m], __ldg(sp + (size_t)m * NT));
+                const float2 z = cmul(v[m], __ldg(sp + 32 * m));
                 v[m] = make_float2(z.x, -z.y);
             }
         }
@@ -964,7 +979,7 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
     line_twiddle(v, a.twN, r, t);
 #pragma unroll
     for (int m = 0; m < E; m++)
-        sts2(seg + q + 256u * m, v[m]);  // row 512 r + t + 16 m
+        sts2(wbase + 16u * RB * m, v[m]);  // row 512 r + t + 16 m
     __syncthreads();
     if constexpr (DSTEP) {
         column_dft(std::true_type());
@@ -973,17 +988,13 @@ __global__ void __launch_bounds__(R * 32, col_r_blocks<R>()) col_pass_r(const Co
         __syncthreads();
 #pragma unroll
         for (int m = 0; m < E; m++)
-            sts2(seg + q + 256u * m, make_float2(v[m].x, -v[m].y));
+            sts2(wbase + 16u * RB * m, make_float2(v[m].x, -v[m].y));
     }
     __syncthreads();
-    // row y's two elements are the 16 bytes at 16 y, column 1 first where
-    // bit 3 of y is set: one 16-byte load per row
 #pragma unroll 4
-    for (int i = 0; i < H / NT; i++) {
-        const int y = threadIdx.x + i * NT;
-        const float4 e = reinterpret_cast<const float4 *>(tile)[y];
-        *reinterpret_cast<float4 *>(C + (size_t)y * W) =
-            (y >> 3) & 1 ? make_float4(e.z, e.w, e.x, e.y) : e;
+    for (int n = threadIdx.x; n < H * PAIRS; n += NT) {
+        const int y = n / PAIRS, u = n % PAIRS;
+        *reinterpret_cast<float4 *>(C + (size_t)y * W + 2 * u) = lds4(base + RB * y + ((16u * u) ^ (8u * TL::f(y))));
     }
 }
 
@@ -997,20 +1008,19 @@ __host__ __device__ __forceinline__ int stored_frequency(int j, int n)
     return R * (j % kLineM) + j / kLineM;
 }
 
-// Launch layout of the line engine's column-pass spectrum: block bx
-// (stored columns 2 bx, 2 bx + 1), register m, thread tid = 32 r + 16 cc + t
-// holds frequency ky = R (t + 16 m) + r of stored column 2 bx + cc.
+// Launch layout of the line engine's column-pass spectrum (see col_pass_r):
+// warp w = pair * R + r, register m, lane l holds frequency
+// ky = R (t + 16 m) + r, t = l >> 1, of stored column 2 pair + (l & 1).
 __global__ void permute_spectrum_r(const float2 *__restrict__ nat, float2 *__restrict__ out, int H, int W, float scale)
 {
-    const int R = H / kLineM, NT = 32 * R;
+    const int R = H / kLineM;
     const size_t total = (size_t)H * W;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int tid = (int)(i % NT);
-        const int m = (int)((i / NT) % 32);
-        const int bx = (int)(i / ((size_t)NT * 32));
-        const int r = tid >> 5, cc = (tid >> 4) & 1, t = tid & 15;
-        const int ky = R * (t + 16 * m) + r;
-        const int kx = stored_frequency(2 * bx + cc, W);
+        const int lane = (int)(i % 32);
+        const int m = (int)((i / 32) % 32);
+        const int w = (int)(i / 1024);
+        const int ky = R * ((lane >> 1) + 16 * m) + w % R;
+        const int kx = stored_frequency(2 * (w / R) + (lane & 1), W);
         const float2 k = nat[(size_t)ky * W + kx];
         out[i] = make_float2(k.x * scale, k.y * scale);
     }
@@ -1200,6 +1210,32 @@ int rl_col_warps(int H, int W, int requested)
 
 size_t rl_spectrum_elems(int H, int W) { return (size_t)H * W; }
 
+// Column-pass warps of a launch.  Four-warp blocks where eight-warp ones would
+// number fewer than 64: twice as many multiprocessors then share the
+// transforms.  Ten iterations of two views (us, 4 / 8 warps): one 512 x 512
+// pair (32 blocks of 8 warps) 519 / 643, two 128 x 128 pairs (8) 234 / 262, two
+// 256 x 256 pairs (32) 390 / 399; but two 512 x 512 pairs (64) 865 / 814 and
+// eight 256 x 256 pairs (128) 523 / 502.  Two warps were never best beyond
+// noise.
+static int launch_col_warps(const RlDims &d, int npairs)
+{
+    if (d.col_auto && d.H <= 1024 && d.col_warps == 8 && d.W / (8 * (32 / warp_fft_lanes(d.H))) * npairs < 64)
+        return 4;
+    return d.col_warps;
+}
+
+// Storage order of the work planes' rows between the passes of a launch.
+static RowSwizzle row_swizzle(const RlDims &d, int npairs)
+{
+    if (d.H != 1024)
+        return RowSwizzle{0, 0};
+    switch (launch_col_warps(d, npairs)) {  // ColTile<1024, 8, 4, 2>::f
+    case 8: return RowSwizzle{ColTile<1024, 8>::sh, 7};
+    case 4: return RowSwizzle{ColTile<1024, 4>::sh, 3};
+    default: return RowSwizzle{ColTile<1024, 2>::sh, 1};
+    }
+}
+
 // Launch of an RL pass with programmatic dependent launch on stream s (the
 // pass's blocks may start while the previous kernel of the stream finishes;
 // the pass waits for it before reading its results).  Falls back to a plain
@@ -1351,13 +1387,14 @@ static void launch_col(const ColArgs &a, int npairs, int cw, int radix_step, cud
     } else {
         constexpr int R = H / kLineM;
         static_assert(H % kLineM == 0 && R >= 3 && R <= 8, "columns above 1024 are 3..8 sub-lines of 512");
-        constexpr size_t smem = sizeof(float2) * 2 * H + 256;  // tile aligned to 256 bytes in the kernel
+        constexpr int FC = kLineColumns;
+        constexpr size_t smem = sizeof(float2) * FC * H + 512;  // tile aligned to 512 bytes in the kernel
         const bool sums = radix_step == kRadixSums;
         auto kern = sums ? col_pass_r<R, false> : col_pass_r<R, true>;
         static unsigned mask[2] = {0, 0};
         configure_smem(kern, smem, mask[sums ? 1 : 0]);
-        dim3 grid(a.W / 2, npairs);
-        launch_pass(kern, grid, dim3(R * 32), smem, s, a);
+        dim3 grid(a.W / FC, npairs);
+        launch_pass(kern, grid, dim3(R * 16 * FC), smem, s, a);
     }
     g_launches++;
 }
@@ -1376,37 +1413,26 @@ static void dispatch_row(const RowArgs &a, cudaStream_t s)
 
 void rl_init(const RlDims &d, const RlBatch &b, const RlTables &t, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
     dispatch_row<ROW_INIT>(a, s);
 }
 
 void rl_divide(const RlDims &d, const RlBatch &b, const RlTables &t, int view, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
     dispatch_row<ROW_DIVIDE>(a, s);
 }
 
 void rl_update(const RlDims &d, const RlBatch &b, const RlTables &t, int view, bool last, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, t.twW};
+    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
     dispatch_row<ROW_UPDATE>(a, s);
 }
 
 void rl_col(const RlDims &d, const RlBatch &b, const RlTables &t, const float2 *spectrum, cudaStream_t s)
 {
     ColArgs a{b.C, spectrum, t.wtwH, d.H, d.W, t.twH};
-    // Four-warp blocks where eight-warp ones would number fewer than 64:
-    // twice as many multiprocessors then share the transforms.  Ten
-    // iterations of two views (us, 4 / 8 warps): one 512 x 512 pair (32 blocks
-    // of 8 warps) 519 / 643, two 128 x 128 pairs (8) 234 / 262, two 256 x 256
-    // pairs (32) 390 / 399; but two 512 x 512 pairs (64) 865 / 814 and eight
-    // 256 x 256 pairs (128) 523 / 502.  Two warps were never best beyond noise.
-    int cw = d.col_warps;
-    if (d.col_auto && d.H <= 1024) {
-        const int G = 32 / warp_fft_lanes(d.H);
-        if (cw == 8 && d.W / (cw * G) * b.npairs < 64)
-            cw = 4;
-    }
+    const int cw = launch_col_warps(d, b.npairs);
     switch (d.H) {
 #define X(N) \
     case N: launch_col<N>(a, b.npairs, cw, d.radix_step, s); break;
