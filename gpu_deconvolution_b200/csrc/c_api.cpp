@@ -235,14 +235,10 @@ int fmvd_b200_transform_device(int bits, const void *d_src, size_t pitch, int w,
         fmvd::report_error("fmvd: invalid arguments to fmvd_b200_transform_device");
         return 1;
     }
-    int *d_status = nullptr;
-    if (!FMVD_CHECK(cudaMallocAsync(&d_status, sizeof(int), (cudaStream_t)stream)))
-        return 1;
-    FMVD_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int), (cudaStream_t)stream));
-    const bool ok = fmvd::resample_device(bits, d_src, pitch, w, h, d, tw, th, z0, nz, h_inverse, d_out, d_outf,
-                                          d_status, (cudaStream_t)stream);
-    FMVD_CHECK(cudaFreeAsync(d_status, (cudaStream_t)stream));
-    return ok ? 0 : 1;
+    return fmvd::resample_device(bits, d_src, pitch, w, h, d, tw, th, z0, nz, h_inverse, d_out, d_outf, nullptr,
+                                 (cudaStream_t)stream)
+               ? 0
+               : 1;
 }
 
 int fmvd_b200_mask_device(float *d_out, int z, int w, int h, int d, float zspacing, int tw, int th, float border,
