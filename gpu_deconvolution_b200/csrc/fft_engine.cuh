@@ -227,9 +227,9 @@ struct DirectDft {
             for (int n = 1; n < R; n++) {
                 float c, s;
                 unit_root<R>((n * k) % R, c, s);
-                // z[n] * (cos - i sin)
-                acc.x += z[n].x * c + z[n].y * s;
-                acc.y += z[n].y * c - z[n].x * s;
+                // z[n] * (cos - i sin), its products fused in one fixed order
+                acc.x = __fadd_rn(acc.x, __fmaf_rn(z[n].x, c, __fmul_rn(z[n].y, s)));
+                acc.y = __fadd_rn(acc.y, __fmaf_rn(z[n].y, c, -__fmul_rn(z[n].x, s)));
             }
             o[k] = acc;
         }

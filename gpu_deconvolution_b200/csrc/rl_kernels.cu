@@ -198,7 +198,22 @@ struct RowWork {
             return (float)reinterpret_cast<const unsigned char *>(row)[sx];
     }
 
-    __device__ __forceinline__ void apply(int x, float2 &v) const
+    // The operands of position x that come from global memory (the estimate;
+    // the two planes' samples), to be requested ahead of the element-wise step.
+    __device__ __forceinline__ float2 fetch(int x) const
+    {
+        if constexpr (MODE == ROW_UPDATE && !EST_S)
+            return est[x];
+        if constexpr (MODE == ROW_DIVIDE && !SMEM) {
+            const int sx = clamp_src(x, d.dataW, d.bxD);
+            return make_float2(sample(src0, sx), has1 ? sample(src1, sx) : 0.f);
+        }
+        return make_float2(0.f, 0.f);
+    }
+
+    __device__ __forceinline__ void apply(int x, float2 &v) const { apply(x, v, fetch(x)); }
+
+    __device__ __forceinline__ void apply(int x, float2 &v, float2 c) const
     {
         if (MODE == ROW_INIT) {
             v = initr0 ? make_float2(__ldcs(initr0 + x), initr1 ? __ldcs(initr1 + x) : 0.f)
@@ -207,28 +222,21 @@ struct RowWork {
         } else if (MODE == ROW_DIVIDE) {
             // q > 1 keeps the divisor in the range where the fast division is
             // within 2 ulp of the IEEE quotient
-            const int sx = clamp_src(x, d.dataW, d.bxD);
-            float a0, a1;
             if constexpr (SMEM) {
-                a0 = lds_sample<BITS>(s_src0, sx);
+                const int sx = clamp_src(x, d.dataW, d.bxD);
+                c.x = lds_sample<BITS>(s_src0, sx);
                 const float s1 = lds_sample<BITS>(s_src1, sx);
-                a1 = has1 ? s1 : 0.f;
-            } else {
-                a0 = sample(src0, sx);
-                a1 = has1 ? sample(src1, sx) : 0.f;
+                c.y = has1 ? s1 : 0.f;
             }
             float2 q = v;
-            q.x = q.x > 1.f ? __fdividef(a0, q.x) : q.x;
-            q.y = q.y > 1.f ? __fdividef(a1, q.y) : q.y;
+            q.x = q.x > 1.f ? __fdividef(c.x, q.x) : q.x;
+            q.y = q.y > 1.f ? __fdividef(c.y, q.y) : q.y;
             v = q;
         } else {
             static_assert(MODE != ROW_UPDATE || SMEM, "the update pass reads its weight row from shared memory");
             const float w = lds_f32(s_w + 4u * clamp_src(x, d.dataW, d.bxW));
-            float2 c;
             if constexpr (EST_S)
                 c = lds_f32x2(s_est + 8u * x);
-            else
-                c = est[x];
             const float2 r = v;
             c.x += w * (c.x * r.x - c.x);
             c.y += w * (c.y * r.y - c.y);
@@ -441,6 +449,11 @@ __global__ void split_estimate_kernel(const float2 *__restrict__ est, int nplane
 __device__ __forceinline__ void sts2(uint32_t addr, float2 v)
 {
     asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts4(uint32_t addr, float4 v)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
 }
 __device__ __forceinline__ float4 lds4(uint32_t addr)
 {
@@ -661,7 +674,13 @@ __device__ __forceinline__ float2 line_coefficient(const float2 *__restrict__ tw
 // (divide) into shared memory after the buffers.
 // DSTEP: the radix-R step as R-point DFTs per position (true) or as each
 // group's weighted sum over all R sub-lines (false); the two schedules give
-// the same transform with different instruction mixes (autotuner knob).
+// the same transform with different instruction mixes (autotuner knob).  With
+// the DFTs the update pass runs the element-wise step between the inverse and
+// the forward one in the same thread: two block barriers and eight
+// shared-memory accesses per point instead of four and twelve (5 to 7 % of a
+// step at R = 3 to 7).  The divide pass and R = 8 keep the separate steps:
+// merged, the compiler fuses other products of their transforms, and samples
+// at a rounding boundary change.
 template <int R, int MODE, int BITS, bool NOOUT, bool SMEM, bool DSTEP>
 __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
 {
@@ -704,11 +723,77 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
             bulk_load(st + rs, work.src1, rb, &sbar[h]);
     }
 
-    // the radix-R step across the row's R groups, v[m] <- sum_j (group j's
-    // v[m]) w_R^(r j): every group puts its sub-line in its buffer (position
-    // n1), then each half-warp of the row takes blocks of 16 positions n1
-    // (block b = r, r + R, ...) and runs the R-point DFT over the R buffers
-    // in place, and every group reads its own buffer back
+    const auto operands_landed = [&]() {
+        if (staged) {
+            if (!mbar_wait(&sbar[h], 0)) {
+                // the copy did not land in time: flag it (the host reports the
+                // batch as failed) and wait once more so no copy is left in flight
+                if (threadIdx.x == 16 * h)
+                    atomicExch(a.b.status, 1);
+                mbar_wait(&sbar[h], 0);
+            }
+            if (MODE == ROW_UPDATE) {
+                work.s_w = smem_u32addr(st);
+            } else {
+                work.s_src0 = smem_u32addr(st);
+                work.s_src1 = work.has1 ? smem_u32addr(st + rs) : work.s_src0;
+            }
+        }
+    };
+    constexpr bool MERGE = DSTEP && MODE != ROW_DIVIDE && R != 8;
+    const bool no_forward = MODE == ROW_UPDATE && !NOOUT && a.last;  // the output is written, nothing follows
+
+    // MERGE: everything between the 512-point transforms.  Every group has its
+    // sub-line in its buffer (position n1); a half-warp takes blocks of 16
+    // positions n1 of its row (block b = r, r + R, ...), and one thread runs the
+    // R-point DFT over the R buffers, which gives it the space positions
+    // n1 + 512 q, the element-wise step on them, and the R-point DFT of the
+    // forward transform, back into the same places.  The next block's operands
+    // from global memory are requested before the current one is worked on.
+    const auto middle = [&]() {
+        float2 c[R];
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            c[q] = work.fetch(q * kLineM + 16 * r + t);
+#pragma unroll 1
+        for (int b = r; b < kLineM / 16; b += R) {
+            float2 z[R], next[R];
+            const int bn = b + R < kLineM / 16 ? b + R : b;
+#pragma unroll
+            for (int q = 0; q < R; q++) {
+                next[q] = work.fetch(q * kLineM + 16 * bn + t);
+                z[q] = MODE == ROW_INIT ? make_float2(0.f, 0.f) : lbuf[q * PF2 + 16 * b + t];
+            }
+            if (MODE != ROW_INIT) {
+                SmallDft<R>::run(z);
+#pragma unroll
+                for (int q = 0; q < R; q++) {
+                    asm volatile("" : "+f"(z[q].x), "+f"(z[q].y));  // rounded here, as where it was stored
+                    z[q].y = -z[q].y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < R; q++) {
+                work.apply(q * kLineM + 16 * b + t, z[q], c[q]);
+                c[q] = next[q];
+            }
+            if (!no_forward) {
+#pragma unroll
+                for (int q = 0; q < R; q++)
+                    asm volatile("" : "+f"(z[q].x), "+f"(z[q].y));
+                SmallDft<R>::run(z);
+#pragma unroll
+                for (int q = 0; q < R; q++)
+                    lbuf[q * PF2 + 16 * b + t] = z[q];
+            }
+        }
+    };
+
+    // The step by itself, v[m] <- sum_j (group j's v[m]) w_R^(r j): every group
+    // puts its sub-line in its buffer (position n1); then (DSTEP) each half-warp
+    // of the row runs the R-point DFT over the R buffers in place and every
+    // group reads its own buffer back, or (!DSTEP) each group sums all R
+    // sub-lines at its own positions.
     const auto line_dft = [&](float2 *v) {
 #pragma unroll
         for (int m = 0; m < E; m++)
@@ -751,10 +836,14 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
     // keeps one copy of the 512-point transform.
     float2 v[E];
     if (MODE == ROW_INIT) {
+        if constexpr (MERGE) {
+            middle();
+        } else {
 #pragma unroll
-        for (int m = 0; m < E; m++) {
-            v[m] = make_float2(0.f, 0.f);
-            work.apply(r * kLineM + t + T * m, v[m]);
+            for (int m = 0; m < E; m++) {
+                v[m] = make_float2(0.f, 0.f);
+                work.apply(r * kLineM + t + T * m, v[m]);
+            }
         }
     } else {
 #pragma unroll
@@ -766,7 +855,15 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
 #pragma unroll 1
     for (int pass = MODE == ROW_INIT ? 1 : 0; pass < 2; pass++) {
         if (pass == 1) {
-            line_dft(v);
+            if constexpr (MERGE) {
+                __syncthreads();
+#pragma unroll
+                for (int m = 0; m < E; m++)
+                    v[m] = buf[t + T * m];
+                __syncwarp();
+            } else {
+                line_dft(v);
+            }
             line_twiddle(v, a.twN, r, t);
         }
         WF::template run_padded<-1>(v, a.tw, buf, t);
@@ -782,28 +879,23 @@ __global__ void __launch_bounds__(R * 32, 16 / R) row_pass_r(const RowArgs a)
             prefetch_l1((const char *)(t < 8 ? work.src0 : work.src1) + (size_t)sx * (BITS == 8 ? 1 : 2));
         }
         line_twiddle(v, a.twN, r, t);
-        line_dft(v);
-        if (staged) {
-            if (!mbar_wait(&sbar[h], 0)) {
-                // the copy did not land in time: flag it (the host reports the
-                // batch as failed) and wait once more so no copy is left in flight
-                if (threadIdx.x == 16 * h)
-                    atomicExch(a.b.status, 1);
-                mbar_wait(&sbar[h], 0);
-            }
-            if (MODE == ROW_UPDATE) {
-                work.s_w = smem_u32addr(st);
-            } else {
-                work.s_src0 = smem_u32addr(st);
-                work.s_src1 = work.has1 ? smem_u32addr(st + rs) : work.s_src0;
-            }
-        }
+        if constexpr (MERGE) {
 #pragma unroll
-        for (int m = 0; m < E; m++) {
-            v[m].y = -v[m].y;
-            work.apply(r * kLineM + t + T * m, v[m]);
+            for (int m = 0; m < E; m++)
+                buf[t + T * m] = v[m];
+            __syncthreads();
+            operands_landed();
+            middle();
+        } else {
+            line_dft(v);
+            operands_landed();
+#pragma unroll
+            for (int m = 0; m < E; m++) {
+                v[m].y = -v[m].y;
+                work.apply(r * kLineM + t + T * m, v[m]);
+            }
         }
-        if (MODE == ROW_UPDATE && !NOOUT && a.last)
+        if (no_forward)
             return;
     }
 #pragma unroll
@@ -890,12 +982,46 @@ __global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_
     if (threadIdx.x == 0)
         bulk_prefetch_l2(sp, (uint32_t)(E * NT * sizeof(float2)));
     pdl_wait();
+    // DSTEP: one thread runs the R-point DFTs of a column pair at a position n1
+    // (rows 512 q + n1), 16 bytes at a time: in place in the tile before the
+    // transforms, and from the tile straight to the plane after them.  (The
+    // first step straight from the plane as well costs 3 to 15 %: its loads are
+    // not asynchronous.)
+    const auto pair_dft = [&](float4 *e) {
+        float2 z0[R], z1[R];
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            z0[q] = make_float2(e[q].x, e[q].y);
+            z1[q] = make_float2(e[q].z, e[q].w);
+        }
+        SmallDft<R>::run(z0);
+        SmallDft<R>::run(z1);
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            e[q] = make_float4(z0[q].x, z0[q].y, z1[q].x, z1[q].y);
+    };
 #pragma unroll 8
     for (int n = threadIdx.x; n < H * PAIRS; n += NT) {
         const int y = n / PAIRS, u = n % PAIRS;
         cp_async16(base + RB * y + ((16u * u) ^ (8u * TL::f(y))), C + (size_t)y * W + 2 * u);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (DSTEP) {
+        __syncthreads();
+#pragma unroll 1
+        for (int n = threadIdx.x; n < kLineM * PAIRS; n += NT) {
+            const int n1 = n / PAIRS, u = n % PAIRS;
+            const uint32_t at = base + RB * n1 + ((16u * u) ^ (8u * TL::f(n1)));
+            float4 e[R];
+#pragma unroll
+            for (int q = 0; q < R; q++)
+                e[q] = lds4(at + kLineM * RB * q);
+            pair_dft(e);
+#pragma unroll
+            for (int q = 0; q < R; q++)
+                sts4(at + kLineM * RB * q, e[q]);
+        }
+    }
     __syncthreads();
     const int t = lane >> 1;
     const uint32_t q = RB * t + 8u * ((2 * pair + (lane & 1)) ^ TL::f(t));
@@ -903,26 +1029,7 @@ __global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_
     const uint32_t seg = base + 512u * RB * r;      // this group's sub-line
     const uint32_t wbase = seg + q, rbase = wbase + 16u * RB * t;
 
-    // The radix-R step of every column in place in the tile: each half-warp
-    // takes blocks of 16 positions n1 of its column (block b = r, r + R, ...)
-    // and runs the R-point DFT over the rows 512 q + n1 (q < R); with CONJ the
-    // results are stored conjugated.  The tile address of row 512 q + 16 b + t
-    // of this column is col + 512 RB q + 16 RB b.
-    const auto column_dft = [&](auto conj_out) {
-#pragma unroll 1
-        for (int b = r; b < kLineM / 16; b += R) {
-            float2 z[R];
-#pragma unroll
-            for (int q = 0; q < R; q++)
-                z[q] = lds2(col + 512u * RB * q + 16u * RB * b);
-            SmallDft<R>::run(z);
-#pragma unroll
-            for (int q = 0; q < R; q++)
-                sts2(col + 512u * RB * q + 16u * RB * b, decltype(conj_out)::value ? make_float2(z[q].x, -z[q].y) : z[q]);
-        }
-    };
-
-    // the other schedule: v[m] = sum_j (row 512 j + t + 16 m of this column) w_R^(r j)
+    // !DSTEP: v[m] = sum_j (row 512 j + t + 16 m of this column) w_R^(r j)
     const auto column_sum = [&](float2 *v) {
 #pragma unroll
         for (int m = 0; m < E; m++)
@@ -950,8 +1057,6 @@ __global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 0) {
             if constexpr (DSTEP) {
-                column_dft(std::false_type());
-                __syncthreads();  // every block of positions has its radix-R step
 #pragma unroll
                 for (int m = 0; m < E; m++)
                     v[m] = lds2(wbase + 16u * RB * m);  // row 512 r + t + 16 m: this group's sub-line
@@ -982,14 +1087,27 @@ __global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_
         sts2(wbase + 16u * RB * m, v[m]);  // row 512 r + t + 16 m
     __syncthreads();
     if constexpr (DSTEP) {
-        column_dft(std::true_type());
-    } else {
-        column_sum(v);
-        __syncthreads();
+#pragma unroll 2
+        for (int n = threadIdx.x; n < kLineM * PAIRS; n += NT) {
+            const int n1 = n / PAIRS, u = n % PAIRS;
+            const uint32_t at = base + RB * n1 + ((16u * u) ^ (8u * TL::f(n1)));
+            float4 e[R];
 #pragma unroll
-        for (int m = 0; m < E; m++)
-            sts2(wbase + 16u * RB * m, make_float2(v[m].x, -v[m].y));
+            for (int q = 0; q < R; q++)
+                e[q] = lds4(at + kLineM * RB * q);
+            pair_dft(e);
+#pragma unroll
+            for (int q = 0; q < R; q++)
+                *reinterpret_cast<float4 *>(C + (size_t)(kLineM * q + n1) * W + 2 * u) =
+                    make_float4(e[q].x, -e[q].y, e[q].z, -e[q].w);
+        }
+        return;
     }
+    column_sum(v);
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < E; m++)
+        sts2(wbase + 16u * RB * m, make_float2(v[m].x, -v[m].y));
     __syncthreads();
 #pragma unroll 4
     for (int n = threadIdx.x; n < H * PAIRS; n += NT) {
