@@ -224,6 +224,7 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
     e->device = dev;
     e->lanes = lanes < 1 ? 1 : (lanes > kMaxLanes ? kMaxLanes : lanes);
     e->pairs_cap = pairs_cap > 0 ? pairs_cap : default_pairs_cap(H, W, e->lanes);
+    e->pairs_auto = pairs_cap <= 0;
     e->spec_elems = rl_spectrum_elems(H, W);
 
     // kernel 2 from the unnormalised kernels, then normalise the caller's kernels
@@ -388,13 +389,29 @@ bool engine_check_status(Engine *e)
     return true;
 }
 
+// Pairs per batch of a run over 'pairs' pairs.  A caller's own batch size is
+// taken as it is; otherwise the pairs are dealt evenly over the lanes, as many
+// batches on each as the work planes need.  Full batches would leave one lane
+// with more (us, six iterations of two views, full / even batches): 32 pairs
+// of 512 x 512 1664 / 1549, 16 pairs 891 / 787, 8 pairs of 1024 x 1024
+// 1825 / 1683, 3 pairs 825 / 727.  Runs of at most 2 M points stay on one lane:
+// two half-size launches no longer fill the GPU each (8 pairs of 512 x 512
+// 534 / 564, 2 pairs of 1024 x 1024 596 / 623, 16 pairs of 256 x 256 318 / 348).
+static int batch_pairs(const Engine *e, int pairs)
+{
+    if (!e->pairs_auto || e->lanes < 2 || (size_t)pairs * e->dims.H * e->dims.W <= ((size_t)2 << 20))
+        return e->pairs_cap;
+    const int rounds = (pairs + e->lanes * e->pairs_cap - 1) / (e->lanes * e->pairs_cap);
+    return (pairs + e->lanes * rounds - 1) / (e->lanes * rounds);
+}
+
 bool engine_run(Engine *e, const void *data, size_t view_stride, void *out, int nplanes, int iterations,
                 float *est_out, cudaStream_t s, const float *init)
 {
     const size_t plane = (size_t)e->dims.dataH * e->dims.dataW;
     const size_t fplane = (size_t)e->dims.H * e->dims.W;
     const size_t es = e->dims.bits == 16 ? 2 : 1;
-    const int per = 2 * e->pairs_cap;
+    const int per = 2 * batch_pairs(e, (nplanes + 1) / 2);
     // more lanes only when there are several batches
     const int nbatches = (nplanes + per - 1) / per;
     const int used = e->lanes < nbatches ? e->lanes : nbatches;
