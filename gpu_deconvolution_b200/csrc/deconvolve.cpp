@@ -123,6 +123,7 @@ struct Streamer {
     cudaStream_t comp[2] = {nullptr, nullptr};
     int nlanes = 1;
     cudaStream_t s_up = nullptr, s_down = nullptr;
+    void *device = nullptr;  // the slots' device buffers, one allocation
 
     bool init(Engine *e, int nstreams)
     {
@@ -146,17 +147,19 @@ struct Streamer {
                   FMVD_CHECK(cudaStreamCreateWithFlags(&s_down, cudaStreamNonBlocking));
         for (int l = 0; l < nlanes && ok; l++)
             ok = FMVD_CHECK(cudaStreamCreateWithFlags(&comp[l], cudaStreamNonBlocking));
+        const size_t in_bytes = sizeof(S) * plane * cap_planes * V;
+        const size_t out_bytes = sizeof(S) * plane * cap_planes;
+        const auto aligned = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+        ok = ok && FMVD_CHECK(cudaMalloc(&device, nslots * (aligned(in_bytes) + aligned(out_bytes))));
         for (int k = 0; k < nslots && ok; k++) {
             Slot &sl = slot[k];
-            const size_t in_bytes = sizeof(S) * plane * cap_planes * V;
-            const size_t out_bytes = sizeof(S) * plane * cap_planes;
+            sl.d_in = (S *)((char *)device + k * (aligned(in_bytes) + aligned(out_bytes)));
+            sl.d_out = (S *)((char *)sl.d_in + aligned(in_bytes));
             sl.h_in = (S *)pinned_acquire(in_bytes);
             sl.in_bytes = sl.h_in ? in_bytes : 0;
             sl.h_out = sl.h_in ? (S *)pinned_acquire(out_bytes) : nullptr;
             sl.out_bytes = sl.h_out ? out_bytes : 0;
-            ok = sl.h_in && sl.h_out && FMVD_CHECK(cudaMalloc(&sl.d_in, in_bytes)) &&
-                 FMVD_CHECK(cudaMalloc(&sl.d_out, out_bytes)) &&
-                 FMVD_CHECK(cudaEventCreateWithFlags(&sl.up, cudaEventDisableTiming)) &&
+            ok = sl.h_in && sl.h_out && FMVD_CHECK(cudaEventCreateWithFlags(&sl.up, cudaEventDisableTiming)) &&
                  FMVD_CHECK(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming)) &&
                  FMVD_CHECK(cudaEventCreateWithFlags(&sl.down, cudaEventDisableTiming));
             if (ok) {  // no clearing: only planes the datasource wrote are uploaded
@@ -170,11 +173,10 @@ struct Streamer {
 
     void release()
     {
+        cudaFree(device);
         for (auto &sl : slot) {
             pinned_release(sl.h_in, sl.in_bytes);
-            cudaFree(sl.d_in);
             pinned_release(sl.h_out, sl.out_bytes);
-            cudaFree(sl.d_out);
             if (sl.up) cudaEventDestroy(sl.up);
             if (sl.done) cudaEventDestroy(sl.done);
             if (sl.down) cudaEventDestroy(sl.down);

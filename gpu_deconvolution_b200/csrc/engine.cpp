@@ -237,20 +237,48 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
         normalize_kernel(h_Kernel[v], kW * kH);
 
     const size_t plane = (size_t)dataH * dataW;
-    bool ok = FMVD_CHECK(cudaMalloc(&e->spec, sizeof(float2) * e->spec_elems * 2 * nViews)) &&
-              FMVD_CHECK(cudaMalloc(&e->weights, sizeof(float) * (size_t)dataH * e->dims.wpitch * nViews)) &&
-              FMVD_CHECK(cudaMalloc(&e->C, sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
-              FMVD_CHECK(cudaMalloc(&e->est, sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
-              FMVD_CHECK(cudaMalloc(&e->twH, sizeof(float2) * H)) && FMVD_CHECK(cudaMalloc(&e->twW, sizeof(float2) * W)) &&
-              FMVD_CHECK(cudaMalloc(&e->wtwH, sizeof(float2) * rl_warp_twiddle_entries(H))) &&
-              FMVD_CHECK(cudaMalloc(&e->wtwW, sizeof(float2) * rl_warp_twiddle_entries(W))) &&
-              FMVD_CHECK(cudaMalloc(&e->status, sizeof(int))) && FMVD_CHECK(cudaMemset(e->status, 0, sizeof(int)));
+    // all device buffers of the plan in one allocation (an allocation and its
+    // release cost 0.1 to 0.3 ms each, a dozen of them more than a small
+    // volume's deconvolution); the plan-time scratch is part of it, over the
+    // work planes, which no run has used yet
+    const size_t points = (size_t)H * W, kn = (size_t)kH * kW;
+    const size_t work_bytes = sizeof(float2) * points * e->pairs_cap;
+    const size_t scratch_bytes = sizeof(float2) * (points + (size_t)kH * W);  // rl_kernel_spectrum's work
+    struct Part {
+        void **p;
+        size_t bytes;
+    };
+    std::vector<Part> parts = {{(void **)&e->spec, sizeof(float2) * e->spec_elems * 2 * nViews},
+                               {(void **)&e->weights, sizeof(float) * (size_t)dataH * e->dims.wpitch * nViews},
+                               {(void **)&e->twH, sizeof(float2) * H},
+                               {(void **)&e->twW, sizeof(float2) * W},
+                               {(void **)&e->wtwH, sizeof(float2) * rl_warp_twiddle_entries(H)},
+                               {(void **)&e->wtwW, sizeof(float2) * rl_warp_twiddle_entries(W)},
+                               {(void **)&e->status, sizeof(int)},
+                               {(void **)&e->est, work_bytes}};
+    for (int l = 0; l + 1 < e->lanes; l++) {
+        parts.push_back({(void **)&e->laneC[l], work_bytes});
+        parts.push_back({(void **)&e->laneEst[l], work_bytes});
+    }
+    parts.push_back({(void **)&e->C, work_bytes});
+    const auto aligned = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (const Part &q : parts)
+        total += aligned(q.bytes);
+    // the scratch starts with C, the last part: spectrum work, kernels, raw weights
+    const size_t scratch = aligned(scratch_bytes) + aligned(sizeof(float) * kn * 2 * nViews) + sizeof(float) * plane * nViews;
+    total += scratch > aligned(work_bytes) ? scratch - aligned(work_bytes) : 0;
+    bool ok = FMVD_CHECK(cudaMalloc(&e->block, total));
+    size_t at = 0;
+    for (const Part &q : parts) {
+        *q.p = ok ? (char *)e->block + at : nullptr;
+        at += aligned(q.bytes);
+    }
+    ok = ok && FMVD_CHECK(cudaMemset(e->status, 0, sizeof(int)));
     if (ok && e->lanes > 1)
         ok = FMVD_CHECK(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
     for (int l = 0; ok && l + 1 < e->lanes; l++)
-        ok = FMVD_CHECK(cudaMalloc(&e->laneC[l], sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
-             FMVD_CHECK(cudaMalloc(&e->laneEst[l], sizeof(float2) * (size_t)H * W * e->pairs_cap)) &&
-             FMVD_CHECK(cudaStreamCreateWithFlags(&e->side[l], cudaStreamNonBlocking)) &&
+        ok = FMVD_CHECK(cudaStreamCreateWithFlags(&e->side[l], cudaStreamNonBlocking)) &&
              FMVD_CHECK(cudaEventCreateWithFlags(&e->ev_join[l], cudaEventDisableTiming));
     if (!ok) {
         engine_destroy(e);
@@ -272,37 +300,31 @@ Engine *engine_create(int bits, int dataH, int dataW, const float *const *h_Weig
              FMVD_CHECK(cudaMemcpy(e->wtwW, wW.data(), sizeof(float2) * wW.size(), cudaMemcpyHostToDevice));
 
         // kernel spectra (FP32 on the device; the twiddle tables are the
-        // float tables above, computed in double on the host and rounded)
-        float2 *work = nullptr;
-        float *d_k = nullptr;
-        ok = ok && FMVD_CHECK(cudaMalloc(&work, sizeof(float2) * ((size_t)H * W + (size_t)kH * W))) &&
-             FMVD_CHECK(cudaMalloc(&d_k, sizeof(float) * kH * kW));
-        for (int v = 0; v < nViews && ok; v++) {
-            for (int which = 0; which < 2 && ok; which++) {
-                const float *src = which == 0 ? h_Kernel[v] : k2[v].data();
-                ok = FMVD_CHECK(cudaMemcpy(d_k, src, sizeof(float) * kH * kW, cudaMemcpyHostToDevice));
-                if (ok) {
-                    rl_kernel_spectrum(d_k, kH, kW, H, W, e->twH, e->twW, work,
-                                       e->spec + e->spec_elems * (2 * v + which), 0);
-                    ok = FMVD_CHECK(cudaGetLastError()) && FMVD_CHECK(cudaDeviceSynchronize());
-                }
-            }
+        // float tables above, computed in double on the host and rounded):
+        // every kernel in one upload, the spectra one after another on the
+        // stream, which also orders their use of the scratch
+        float2 *work = e->C;
+        float *d_k = (float *)((char *)e->C + aligned(scratch_bytes));
+        std::vector<float> kernels(kn * 2 * nViews);
+        for (int v = 0; v < nViews; v++) {
+            memcpy(&kernels[kn * (2 * v)], h_Kernel[v], sizeof(float) * kn);
+            memcpy(&kernels[kn * (2 * v + 1)], k2[v].data(), sizeof(float) * kn);
         }
-        cudaFree(work);
-        cudaFree(d_k);
+        ok = ok && FMVD_CHECK(cudaMemcpy(d_k, kernels.data(), sizeof(float) * kernels.size(), cudaMemcpyHostToDevice));
+        for (int i = 0; i < 2 * nViews && ok; i++) {
+            rl_kernel_spectrum(d_k + kn * i, kH, kW, H, W, e->twH, e->twW, work, e->spec + e->spec_elems * i, 0);
+            ok = FMVD_CHECK(cudaGetLastError());
+        }
     }
 
     // weights normalised over views
     if (ok) {
-        float *raw = nullptr;
-        ok = FMVD_CHECK(cudaMalloc(&raw, sizeof(float) * plane * nViews));
+        float *raw = (float *)((char *)e->C + aligned(scratch_bytes) + aligned(sizeof(float) * kn * 2 * nViews));
         for (int v = 0; v < nViews && ok; v++)
             ok = FMVD_CHECK(cudaMemcpy(raw + plane * v, h_Weights[v], sizeof(float) * plane, cudaMemcpyHostToDevice));
-        if (ok) {
+        if (ok)
             rl_normalize_weights(e->dims, raw, e->weights, 0);
-            ok = FMVD_CHECK(cudaGetLastError()) && FMVD_CHECK(cudaDeviceSynchronize());
-        }
-        cudaFree(raw);
+        ok = ok && FMVD_CHECK(cudaGetLastError()) && FMVD_CHECK(cudaDeviceSynchronize());
     }
     if (!ok) {
         engine_destroy(e);
@@ -315,18 +337,8 @@ void engine_destroy(Engine *e)
 {
     if (!e)
         return;
-    cudaFree(e->spec);
-    cudaFree(e->weights);
-    cudaFree(e->C);
-    cudaFree(e->est);
-    cudaFree(e->twH);
-    cudaFree(e->twW);
-    cudaFree(e->wtwH);
-    cudaFree(e->wtwW);
-    cudaFree(e->status);
+    cudaFree(e->block);
     for (int l = 0; l + 1 < kMaxLanes; l++) {
-        cudaFree(e->laneC[l]);
-        cudaFree(e->laneEst[l]);
         if (e->side[l])
             cudaStreamDestroy(e->side[l]);
         if (e->ev_join[l])

@@ -28,6 +28,7 @@ struct Engine {
     int kH, kW;
     int pairs_cap;          // plane pairs per batch
     bool pairs_auto;        // the caller left the batch size to the library
+    void *block;            // the one allocation that holds every device buffer below
     int device;
     size_t spec_elems;      // complex values per kernel spectrum (launch layout)
     float2 *spec;           // V x 2 spectra: [v][0] kernel 1, [v][1] kernel 2
