@@ -205,11 +205,11 @@ def peak_hbm():
 # (22.1 MB per view update; the batch's work planes stay in L2).
 DRAM_BYTES_PER_PADDED_VOXEL_VIEW_UPDATE = 3.52
 # Thread instructions of the same four passes per padded voxel (the same
-# capture's smsp__inst_executed.sum x 32 / padded voxels: 38.62 M warp
+# batch shape's sm__inst_executed.sum x 32 / padded voxels: 36.92 M warp
 # instructions per view update of the 6-plane batch).  With one warp
 # instruction per SM sub-partition per cycle (148 SMs x 4 x 32 lanes x clock)
 # this gives the issue-bound ceiling of the passes.
-THREAD_INSTR_PER_PADDED_VOXEL_VIEW_UPDATE = 196.3
+THREAD_INSTR_PER_PADDED_VOXEL_VIEW_UPDATE = 187.9
 
 
 def dist_setup(n):
