@@ -945,13 +945,12 @@ __device__ __forceinline__ void col_fft_512(float2 *v, const TW &tw, uint32_t wb
 // Column pass for H = R * 512: R warps per column pair (lane l of the warp
 // (r, pair) is in group r of column 2 pair + (l & 1)), four columns per block,
 // so that a row of the tile is a whole 32-byte sector and comes by 16-byte
-// copies.  With two columns per block, filled eight bytes at a time, a launch
-// of one 2560 x 2560 pair took 79 us and 510 MB of L2 traffic, now 66 us and
-// 370 MB (1536 x 1536: 32 -> 24 us);
-// ten iterations of 1400 x 1400 x 12 went from 17.7 to 14.4 ms.  Against two
-// columns filled by 16-byte copies: 13 % faster at R = 3, 9 % at 4, 11 % at 5,
-// 3 % at 6, 5 % at 8, 0.6 % slower at 7.  Bound by its two block barriers per
-// radix-R step, issue and L2 latency.
+// copies.  A launch of one 2560 x 2560 pair takes 62 us and 366 MB of L2
+// traffic (79 us and 510 MB with two columns per block, filled eight bytes at a
+// time), one of 1536 x 1536 23 us (32 us).  Against two columns filled by
+// 16-byte copies the step is 13 % faster at R = 3, 9 % at 4, 11 % at 5, 3 % at
+// 6, 5 % at 8, 0.6 % slower at 7.  Bound by its block barriers, shared-memory
+// accesses and L2 latency (43 % issue active).
 // Spectrum in launch layout: warp w = pair * R + r of the plane, register m,
 // lane l at spec[(w * 32 + m) * 32 + l].
 constexpr int kLineColumns = 4;
