@@ -22,12 +22,14 @@
 #include <stdio.h>
 #include <string.h>
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <thread>
 #include <type_traits>
 #include <vector>
 
 #include "fmvd_internal.h"
+#include "smem_opt_in.h"
 #include "transform_kernels.h"
 
 namespace fmvd {
@@ -39,6 +41,9 @@ constexpr int TX = 32, TY = 8;  // target tile
 #define FMVD_RESAMPLE_STACK 16
 #endif
 constexpr int kMaxStack = FMVD_RESAMPLE_STACK;  // target planes per CTA, at most
+// bytes of a brick, at most: a stack of target planes, and a tile of the maps
+// about the y axis
+constexpr size_t kStackSmem = 96 * 1024, kYrotSmem = 54 * 1024;
 
 struct Mat {
     float m[12];
@@ -543,12 +548,12 @@ bool resample_device(int bits, const void *d_src, size_t pitch, int w, int h, in
     int depth = 0;
     if (M.m[1] == 0.f && M.m[9] == 0.f && M.m[4] == 0.f && M.m[6] == 0.f)
         for (int k = kYrotRows; k >= 8 && !depth; k /= 2)
-            depth = box_fits(32, k, kYrotPlanes, 54 * 1024) ? k : 0;
+            depth = box_fits(32, k, kYrotPlanes, kYrotSmem) ? k : 0;
     const bool yrot = depth > 0;
     // any other map takes the deepest stack of 16, 8, 4, 2 or 1 target planes
     // whose box fits
     for (int k = kMaxStack; k >= 1 && !depth; k /= 2)
-        depth = box_fits(TX, TY, k, 96 * 1024) ? k : 0;
+        depth = box_fits(TX, TY, k, kStackSmem) ? k : 0;
 
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));
@@ -571,33 +576,30 @@ bool resample_device(int bits, const void *d_src, size_t pitch, int w, int h, in
     const int mode = (d_out ? kOutSamples : 0) | (d_outf ? kOutFloat : 0);
     if (mode == 0)
         return true;
-    const auto launch = [&](auto general, auto rotated, auto *src_typed, auto *out_typed) {
-        const Source<std::remove_const_t<std::remove_pointer_t<decltype(src_typed)>>> v{src_typed, w, h, d, pitch,
-                                                                                       box[0], box[1], box[2]};
-        auto kern = yrot ? rotated : general;
+    const auto launch = [&](auto bits_c, auto out_c, const auto *src, auto *out) {
+        constexpr int B = decltype(bits_c)::value, OUT = decltype(out_c)::value;
+        using S = std::remove_pointer_t<decltype(out)>;
+        static std::atomic<unsigned long long> tma_devices{0}, yrot_devices{0};
+        auto kern = yrot ? resample_yrot<S, B, OUT> : resample_tma<S, B, OUT>;
+        if (!FMVD_CHECK(allow_smem(kern, yrot ? kYrotSmem : kStackSmem, yrot ? yrot_devices : tma_devices)))
+            return false;
+        const Source<S> v{src, w, h, d, pitch, box[0], box[1], box[2]};
         const dim3 grid = yrot ? dim3((tw + 31) / 32, (th + depth - 1) / depth, (nz + kYrotPlanes - 1) / kYrotPlanes)
                                : dim3((tw + TX - 1) / TX, (th + TY - 1) / TY, (nz + depth - 1) / depth);
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, TX * TY, smem, s>>>(tmap, v, tw, th, z0, nz, depth, M, out_typed, d_outf, d_status);
+        kern<<<grid, TX * TY, smem, s>>>(tmap, v, tw, th, z0, nz, depth, M, out, d_outf, d_status);
         rl_count_launch(1);
+        return FMVD_CHECK(cudaGetLastError());
     };
-    const auto launch_mode = [&](auto bits_c, auto *src_typed, auto *out_typed) {
-        constexpr int B = decltype(bits_c)::value;
-        using S = std::remove_pointer_t<decltype(out_typed)>;
+    const auto launch_mode = [&](auto bits_c, const auto *src, auto *out) {
         if (mode == kOutSamples)
-            launch(resample_tma<S, B, kOutSamples>, resample_yrot<S, B, kOutSamples>, src_typed, out_typed);
-        else if (mode == kOutFloat)
-            launch(resample_tma<S, B, kOutFloat>, resample_yrot<S, B, kOutFloat>, src_typed, out_typed);
-        else
-            launch(resample_tma<S, B, kOutSamples | kOutFloat>, resample_yrot<S, B, kOutSamples | kOutFloat>, src_typed,
-                   out_typed);
+            return launch(bits_c, std::integral_constant<int, kOutSamples>(), src, out);
+        if (mode == kOutFloat)
+            return launch(bits_c, std::integral_constant<int, kOutFloat>(), src, out);
+        return launch(bits_c, std::integral_constant<int, kOutSamples | kOutFloat>(), src, out);
     };
     if (bits == 16)
-        launch_mode(std::integral_constant<int, 16>(), (const unsigned short *)d_src, (unsigned short *)d_out);
-    else
-        launch_mode(std::integral_constant<int, 8>(), (const unsigned char *)d_src, (unsigned char *)d_out);
-    return FMVD_CHECK(cudaGetLastError());
+        return launch_mode(std::integral_constant<int, 16>(), (const unsigned short *)d_src, (unsigned short *)d_out);
+    return launch_mode(std::integral_constant<int, 8>(), (const unsigned char *)d_src, (unsigned char *)d_out);
 }
 
 bool mask_device(float *d_out, int z, int w, int h, int d, float zspacing, int tw, int th, float border,
