@@ -23,7 +23,9 @@
 // box with a one-pixel border.
 //
 // Every mbarrier wait is bounded: on a timeout the CTA records an error in
-// *status and finishes without hanging.
+// *status and finishes without hanging.  A role that runs on a whole warp
+// leaves its loops with all lanes together (warp_wait, warp_sees): its MMAs,
+// commits and tensor-memory loads wait for every lane of the warp.
 #include "fmvd_internal.h"
 #include "tma_util.cuh"
 #include "umma.cuh"
@@ -48,6 +50,15 @@ __device__ __forceinline__ void tap_offset(int taps, int t, int &dy, int &dx)
         dy = dx = 0;
     }
 }
+
+// Bounded wait of a whole, converged warp: lanes poll for themselves, and one
+// that gave up decides for all.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, umma::bar_wait(bar, parity));
+}
+// Whether any lane of a whole, converged warp sees the flag another role raises.
+__device__ __forceinline__ bool warp_sees(int flag) { return __any_sync(0xffffffffu, flag); }
 
 // Sixteen bf16 values as floats (vec: p on a 32-byte boundary).
 __device__ __forceinline__ void load16(const bf16 *p, int vec, float (&f)[16])
@@ -227,9 +238,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- MMA issue
         const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
         int gk = 0, it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
+        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
             const int ab = it & 1;
-            if (it >= 2 && !umma::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+            if (it >= 2 && !warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
             const uint32_t acc = tmem + ab * C::ACC_COLS;
             for (int kb = 0; kb < nk; kb++, gk++) {
                 const int s = gk % C::STAGES, round = gk / C::STAGES;
-                if (!umma::bar_wait(&full[s], round & 1)) {
+                if (!warp_wait(&full[s], round & 1)) {
                     fail_sh = 1;
                     break;
                 }
@@ -256,9 +267,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- epilogue: warp w owns accumulator rows 32w..32w+31
         const int row = warp * 32 + lane;
         int it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
+        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
             const int ab = it & 1;
-            if (!umma::bar_wait(&acc_full[ab], (it >> 1) & 1)) {
+            if (!warp_wait(&acc_full[ab], (it >> 1) & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -391,12 +402,12 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- MMA issue
         const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
         const umma::Desc bd = umma::make_desc(umma::smem_addr(wsm), 16, 8 * C::R, C::R);
-        if (!umma::bar_wait(&wfull, 0))
+        if (!warp_wait(&wfull, 0))
             fail_sh = 1;
         int gs = 0, it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++, gs += NB) {
+        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++, gs += NB) {
             const int ab = it & 1;
-            if (it >= 2 && !umma::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+            if (it >= 2 && !warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
 #pragma unroll
             for (int cb = 0; cb < NB; cb++) {
                 const int s = (gs + cb) % C::SLOTS, round = (gs + cb) / C::SLOTS;
-                ok = ok && umma::bar_wait(&full[s], round & 1);
+                ok = ok && warp_wait(&full[s], round & 1);
                 ad[cb] = umma::make_desc(umma::smem_addr(slots) + s * C::SLOT, 16, kBoxW * C::R, C::R);
             }
             if (!ok) {
@@ -432,9 +443,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- epilogue: warp w owns accumulator rows 32w..32w+31
         const int row = warp * 32 + lane;
         int it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !fail_sh; tile += gridDim.x, it++) {
+        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
             const int ab = it & 1;
-            if (!umma::bar_wait(&acc_full[ab], (it >> 1) & 1)) {
+            if (!warp_wait(&acc_full[ab], (it >> 1) & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -450,6 +461,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
                 umma::tmem_ld16(trow + c0, v);
                 if (y < g.H)
                     epilogue16(g, pix, c0, v);
+                __syncwarp();  // rows past the image skip the stores
             }
             umma::tc_fence_before();
             __syncwarp();
@@ -578,7 +590,7 @@ __global__ void __launch_bounds__(128, 1)
         const uint32_t idesc = umma::make_idesc(128, BN, 1, 1);
         for (int k = 0; k < nk; k++) {
             const int s = k % C::STAGES, round = k / C::STAGES;
-            if (!umma::bar_wait(&full[s], round & 1)) {
+            if (!warp_wait(&full[s], round & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -607,7 +619,7 @@ __global__ void __launch_bounds__(128, 1)
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int k = 0; k < nk; k++) {
             const int s = k % C::STAGES, round = k / C::STAGES;
-            if (!umma::bar_wait(&full[s], round & 1)) {
+            if (!warp_wait(&full[s], round & 1)) {
                 fail_sh = 1;
                 break;
             }
@@ -640,7 +652,8 @@ __global__ void __launch_bounds__(128, 1)
     __syncwarp();
 
     // accumulator rows are TMEM lanes (warp w: lanes 32w..)
-    const bool got = umma::bar_wait(&done, 0);
+    if (!warp_wait(&done, 0))
+        fail_sh = 1;
     umma::tc_fence_after();
     const int row = warp * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
@@ -660,10 +673,10 @@ __global__ void __launch_bounds__(128, 1)
                 atomicAdd(dst + (size_t)i * TAPS * g.cin, v[i]);
         }
     }
-    if (threadIdx.x == 0 && (!got || fail_sh) && g.status)
-        atomicExch(g.status, 1);
     umma::tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0 && fail_sh && g.status)
+        atomicExch(g.status, 1);
     if (warp == 0)
         umma::tmem_dealloc(tmem, C::TCOLS);
 }
