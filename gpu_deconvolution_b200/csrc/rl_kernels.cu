@@ -1333,20 +1333,22 @@ size_t rl_spectrum_elems(int H, int W) { return (size_t)H * W; }
 // pair (32 blocks of 8 warps) 519 / 643, two 128 x 128 pairs (8) 234 / 262, two
 // 256 x 256 pairs (32) 390 / 399; but two 512 x 512 pairs (64) 865 / 814 and
 // eight 256 x 256 pairs (128) 523 / 502.  Two warps were never best beyond
-// noise.
+// noise.  Not for 1024 rows, where a warp is one column and four of them read
+// 32 bytes of a row instead of 64 (five iterations of two views, 4 / 8 warps): one 1024 x 256 pair 291 / 239, four 1024 x 64 pairs 291 / 236, one
+// 1024 x 128 pair 247 / 236.
 static int launch_col_warps(const RlDims &d, int npairs)
 {
-    if (d.col_auto && d.H <= 1024 && d.col_warps == 8 && d.W / (8 * (32 / warp_fft_lanes(d.H))) * npairs < 64)
+    if (d.col_auto && d.H < 1024 && d.col_warps == 8 && d.W / (8 * (32 / warp_fft_lanes(d.H))) * npairs < 64)
         return 4;
     return d.col_warps;
 }
 
-// Storage order of the work planes' rows between the passes of a launch.
-static RowSwizzle row_swizzle(const RlDims &d, int npairs)
+// Storage order of the work planes' rows between the passes.
+static RowSwizzle row_swizzle(const RlDims &d)
 {
     if (d.H != 1024)
         return RowSwizzle{0, 0};
-    switch (launch_col_warps(d, npairs)) {  // ColTile<1024, 8, 4, 2>::f
+    switch (d.col_warps) {  // ColTile<1024, 8, 4, 2>::f
     case 8: return RowSwizzle{ColTile<1024, 8>::sh, 7};
     case 4: return RowSwizzle{ColTile<1024, 4>::sh, 3};
     default: return RowSwizzle{ColTile<1024, 2>::sh, 1};
@@ -1530,19 +1532,19 @@ static void dispatch_row(const RowArgs &a, cudaStream_t s)
 
 void rl_init(const RlDims &d, const RlBatch &b, const RlTables &t, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
+    RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, row_swizzle(d), t.twW};
     dispatch_row<ROW_INIT>(a, s);
 }
 
 void rl_divide(const RlDims &d, const RlBatch &b, const RlTables &t, int view, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
+    RowArgs a{d, b, t.wtwW, view, 0, 0, 0, row_swizzle(d), t.twW};
     dispatch_row<ROW_DIVIDE>(a, s);
 }
 
 void rl_update(const RlDims &d, const RlBatch &b, const RlTables &t, int view, bool last, cudaStream_t s)
 {
-    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, row_swizzle(d, b.npairs), t.twW};
+    RowArgs a{d, b, t.wtwW, view, last ? 1 : 0, 0, 0, row_swizzle(d), t.twW};
     dispatch_row<ROW_UPDATE>(a, s);
 }
 
