@@ -954,12 +954,22 @@ __device__ __forceinline__ void col_fft_512(float2 *v, const TW &tw, uint32_t wb
 // Spectrum in launch layout: warp w = pair * R + r of the plane, register m,
 // lane l at spec[(w * 32 + m) * 32 + l].
 constexpr int kLineColumns = 4;
-// Resident blocks per SM
+// Resident blocks per SM, which cap the registers of a thread.  A launch of at
+// most one block per multiprocessor has nothing to share an SM with, and takes
+// the kernel compiled for one (R = 3 to 5: 204 to 255 registers instead of 102
+// to 128, so more loads in flight per thread; from R = 6 on they are the same).
+// Five iterations of two views (us, shared / one block, and two columns per
+// block as before): one pair of 1536 x 256 (64 blocks) 437 / 280, 435; three of
+// 1536 x 64 (48) 407 / 269, 366; one of 2048 x 512 (128) 528 / 429, 696; one of
+// 2560 x 512 (128) 657 / 486, 771; one of 1536 x 128 (32) 317 / 290, 248.
+// Beyond a block per SM the shared one is as good or better: three pairs of
+// 2048 x 256 (192) 502 / 544, two of 2048 x 512 (256) 576 / 632, three of
+// 2560 x 256 (192) 620 / 669.
 template <int R>
 __host__ __device__ constexpr int col_r_blocks() { return R == 3 ? 3 : R <= 5 ? 2 : 1; }
 
-template <int R, bool DSTEP>
-__global__ void __launch_bounds__(R * 16 * kLineColumns, col_r_blocks<R>()) col_pass_r(const ColArgs a)
+template <int R, bool DSTEP, int BLOCKS>
+__global__ void __launch_bounds__(R * 16 * kLineColumns, BLOCKS) col_pass_r(const ColArgs a)
 {
     using WF = WarpFft<kLineM>;
     static_assert(WF::T == 16 && WF::E == 32, "sub-lines are 512-point half-warp transforms");
@@ -1508,10 +1518,12 @@ static void launch_col(const ColArgs &a, int npairs, int cw, int radix_step, cud
         static_assert(H % kLineM == 0 && R >= 3 && R <= 8, "columns above 1024 are 3..8 sub-lines of 512");
         constexpr int FC = kLineColumns;
         constexpr size_t smem = sizeof(float2) * FC * H + 512;  // tile aligned to 512 bytes in the kernel
-        const bool sums = radix_step == kRadixSums;
-        auto kern = sums ? col_pass_r<R, false> : col_pass_r<R, true>;
-        static unsigned mask[2] = {0, 0};
-        configure_smem(kern, smem, mask[sums ? 1 : 0]);
+        const bool sums = radix_step == kRadixSums, few = a.W / FC * npairs <= kSms;
+        constexpr int B = col_r_blocks<R>();
+        auto kern = sums ? (few ? col_pass_r<R, false, 1> : col_pass_r<R, false, B>)
+                         : (few ? col_pass_r<R, true, 1> : col_pass_r<R, true, B>);
+        static unsigned mask[4] = {0, 0, 0, 0};
+        configure_smem(kern, smem, mask[(sums ? 2 : 0) + (few ? 1 : 0)]);
         dim3 grid(a.W / FC, npairs);
         launch_pass(kern, grid, dim3(R * 16 * FC), smem, s, a);
     }
