@@ -544,9 +544,16 @@ bool resample_device(int bits, const void *d_src, size_t pitch, int w, int h, in
         return box[0] <= 256 && box[1] <= 256 && box[2] <= 256 && smem <= limit;
     };
     // a rotation about y walks down rows: the deepest of 32, 16 or 8 whose
-    // brick leaves room for four blocks on a multiprocessor
+    // brick leaves room for four blocks on a multiprocessor.  Not where a target
+    // row is many source rows further, so that no row serves two voxels, and
+    // neighbouring voxels also lie in different source planes of the brick: 64
+    // planes of 420 x 400 into 200 of them turned by 90 degrees, plane distance
+    // 3, rows walked / stacks of planes (us): 16 bits 142 / 108 at 4.5 source
+    // rows, 178 / 117 at 6, 230 / 142 at 8; 8 bits 104 / 114 at 4.5, 111 / 115
+    // at 5, 125 / 115 at 6, 156 / 121 at 8
+    const bool about_y = M.m[1] == 0.f && M.m[9] == 0.f && M.m[4] == 0.f && M.m[6] == 0.f;
     int depth = 0;
-    if (M.m[1] == 0.f && M.m[9] == 0.f && M.m[4] == 0.f && M.m[6] == 0.f)
+    if (about_y && (fabsf(M.m[5]) <= (bits == 16 ? 4.f : 5.f) || fabsf(M.m[8]) <= 0.25f))
         for (int k = kYrotRows; k >= 8 && !depth; k /= 2)
             depth = box_fits(32, k, kYrotPlanes, kYrotSmem) ? k : 0;
     const bool yrot = depth > 0;
