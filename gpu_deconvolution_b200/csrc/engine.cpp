@@ -402,16 +402,23 @@ bool engine_check_status(Engine *e)
 }
 
 // Pairs per batch of a run over 'pairs' pairs.  A caller's own batch size is
-// taken as it is; otherwise the pairs are dealt evenly over the lanes, as many
-// batches on each as the work planes need.  Full batches would leave one lane
-// with more (us, six iterations of two views, full / even batches): 32 pairs
-// of 512 x 512 1664 / 1549, 16 pairs 891 / 787, 8 pairs of 1024 x 1024
-// 1825 / 1683, 3 pairs 825 / 727.  Runs of at most 2 M points stay on one lane:
-// two half-size launches no longer fill the GPU each (8 pairs of 512 x 512
-// 534 / 564, 2 pairs of 1024 x 1024 596 / 623, 16 pairs of 256 x 256 318 / 348).
+// taken as it is, and a run whose column passes are one wave of blocks is left in
+// full batches: launches of half the size would each leave multiprocessors
+// idle.  Past that the pairs are dealt evenly over the lanes, as many batches on
+// each as the work planes need: one launch's partly filled last wave runs beside
+// the other lane's, and no lane has more than the others.  Four or five
+// iterations of two views (us, one lane / dealt), the last size of a wave and
+// the first beyond it: 512 x 256 18 pairs 442 / 501, 19 533 / 515; 1024 x 256 9
+// 469 / 535, 10 586 / 562; 1024 x 64 36 494 / 569, 38 603 / 600; 256 x 512 18
+// 454 / 506, 19 548 / 530; 128 x 1024 18 440 / 499, 19 533 / 508; 128 x 1536 12
+// 633 / 646, 13 699 / 677; 1536 x 64 27 664 / 685, 28 782 / 745; 2048 x 128 9
+// 573 / 651, 10 747 / 708; 2560 x 64 18 719 / 756, 19 923 / 835; 3584 x 128 4
+// 610 / 673, 5 962 / 843; 4096 x 128 4 586 / 673, 5 942 / 788.  512 x 512 gains
+// later: 9 pairs 454 / 605, 10 594 / 628, 12 513 / 506, 16 641 / 576.
 static int batch_pairs(const Engine *e, int pairs)
 {
-    if (!e->pairs_auto || e->lanes < 2 || (size_t)pairs * e->dims.H * e->dims.W <= ((size_t)2 << 20))
+    if (!e->pairs_auto || e->lanes < 2 ||
+        (size_t)pairs * e->dims.H * e->dims.W <= rl_wave_points(e->dims.H))
         return e->pairs_cap;
     const int rounds = (pairs + e->lanes * e->pairs_cap - 1) / (e->lanes * e->pairs_cap);
     return (pairs + e->lanes * rounds - 1) / (e->lanes * rounds);

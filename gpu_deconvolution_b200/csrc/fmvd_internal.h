@@ -70,7 +70,7 @@ int default_pairs_cap(int H, int W, int lanes = 1);
 // Deconvolve nplanes planes resident on the device.  View v, plane z of the
 // input is at data + (v * view_stride + z * plane) samples; plane z of the
 // output at out + z * plane.  est_out (optional) receives nplanes float
-// planes of H x W.  Planes are processed in batches of 2 * pairs_cap.
+// planes of H x W.  Planes are processed in batches of at most 2 * pairs_cap.
 // init (optional): nplanes float planes of H x W to start from instead of the
 // reference's constant 10 * nViews; running k iterations from the estimate
 // that j iterations returned gives the result of j + k iterations.

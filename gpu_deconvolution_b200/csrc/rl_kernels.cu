@@ -1542,6 +1542,25 @@ static void dispatch_row(const RowArgs &a, cudaStream_t s)
     }
 }
 
+size_t rl_wave_points(int H)
+{
+    // up to 1024 rows two blocks of 256 threads and 32 values each per SM (at
+    // 512 and 1024 rows; shorter columns, with 16 values or fewer per thread,
+    // take two waves of shorter blocks to the same line)
+    size_t per_sm = 2 * 256 * 32;
+    switch (H) {
+#define X(N) \
+    case N: \
+        if constexpr (N > 1024) \
+            per_sm = (size_t)col_r_blocks<N / kLineM>() * kLineColumns * N; \
+        break;
+        FMVD_FOR_EACH_LENGTH(X)
+#undef X
+    default: break;
+    }
+    return kSms * per_sm;
+}
+
 void rl_init(const RlDims &d, const RlBatch &b, const RlTables &t, cudaStream_t s)
 {
     RowArgs a{d, b, t.wtwW, 0, 0, 0, 0, row_swizzle(d), t.twW};

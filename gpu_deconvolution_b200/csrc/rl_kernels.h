@@ -67,6 +67,9 @@ int rl_warp_twiddle_entries(int n);
 // Column-pass warps per block for an H x W plane: 'requested' (2, 4 or 8)
 // when the plane allows it, the widest allowed when 0, -1 when not allowed.
 int rl_col_warps(int H, int W, int requested);
+// Points whose column pass is one wave of blocks: what a launch may hold before
+// its blocks no longer run at once.
+size_t rl_wave_points(int H);
 
 bool rl_length_supported(int n);
 // Number of kernel launches this library has issued (all kernels).
