@@ -27,6 +27,7 @@
 // leaves its loops with all lanes together (warp_wait, warp_sees): its MMAs,
 // commits and tensor-memory loads wait for every lane of the warp.
 #include "fmvd_internal.h"
+#include "smem_opt_in.h"
 #include "tma_util.cuh"
 #include "umma.cuh"
 #include "unet.h"
@@ -34,6 +35,7 @@
 #include <cuda_bf16.h>
 #include <stdio.h>
 #include <algorithm>
+#include <atomic>
 
 namespace fmvd {
 namespace unet {
@@ -734,20 +736,15 @@ void pixel_box(int W, int count, int &bw, int &bh)
     bh = count / bw;
 }
 
-// Opts a kernel in to its dynamic shared memory (once per process; the
-// devices of a process are alike) and reads the multiprocessor count.
+// Opts a kernel in to its dynamic shared memory on the current device and reads
+// the device's multiprocessor count.
 template <typename K>
-bool configure(K kern, uint32_t smem, int &sms)
+bool configure(K kern, uint32_t smem, std::atomic<unsigned long long> &devices, int &sms)
 {
-    if (sms)
-        return true;
-    int dev = 0, n = 0;
-    if (!FMVD_CHECK(cudaGetDevice(&dev)) ||
-        !FMVD_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) ||
-        !FMVD_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
-        return false;
-    sms = n;
-    return true;
+    int dev = 0;
+    return FMVD_CHECK(cudaGetDevice(&dev)) &&
+           FMVD_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) &&
+           FMVD_CHECK(allow_smem(kern, smem, devices));
 }
 
 template <int CB, int BN>
@@ -756,8 +753,9 @@ bool launch_persistent(const CUtensorMap &ta, const CUtensorMap &tb, const GemmA
 {
     using C = PersistCfg<CB, BN>;
     auto k = conv_gemm_persistent<CB, BN>;
-    static int sms = 0;
-    if (!configure(k, C::SMEM, sms))
+    static std::atomic<unsigned long long> devices{0};
+    int sms = 0;
+    if (!configure(k, C::SMEM, devices, sms))
         return false;
     // CTAs per SM: tensor memory (512 columns) and shared memory allow
     const int by_tmem = 512 / C::TCOLS;
@@ -793,8 +791,9 @@ bool launch_halo(const CUtensorMap &ta, const CUtensorMap &tb, const GemmArgs &g
 {
     using C = HaloCfg<CB, NB, BN>;
     auto k = conv_halo<CB, NB, BN>;
-    static int sms = 0;
-    if (!configure(k, C::SMEM, sms))
+    static std::atomic<unsigned long long> devices{0};
+    int sms = 0;
+    if (!configure(k, C::SMEM, devices, sms))
         return false;
     const int ntiles = g.N * ((g.H + kTileH - 1) / kTileH) * (g.W / kTileW);
     // CTAs per SM: tensor memory (512 columns), shared memory (228 KB, 1 KB of
@@ -826,8 +825,9 @@ bool launch_wgrad(const CUtensorMap &tx, const CUtensorMap &tg, const GemmArgs &
 {
     using C = WgradCfg<CB, GROUPS, PACK, BN, TAPS>;
     auto k = conv_wgrad_kernel<CB, GROUPS, PACK, BN, TAPS>;
-    static int sms = 0;
-    if (!configure(k, C::SMEM, sms))
+    static std::atomic<unsigned long long> devices{0};
+    int sms = 0;
+    if (!configure(k, C::SMEM, devices, sms))
         return false;
     const int ntiles = g.N * ((g.H + kGradH - 1) / kGradH) * ((g.W + kGradW - 1) / kGradW);
     // pixels per CTA: a bounded accumulation (see the kernel), at least 8 tiles
