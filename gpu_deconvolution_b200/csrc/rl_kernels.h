@@ -18,7 +18,7 @@ struct RlDims {
     int byD, bxD;
     int byW, bxW;
     int col_warps;       // column-pass warps per block (warp engine, H <= 1024)
-    int col_auto;        // the caller left col_warps to the library: narrower blocks for few planes
+    int col_auto;        // the caller left col_warps to the library: narrower blocks for few planes below 1024 rows
     int wpitch;          // floats per stored weight row: dataW rounded up to a multiple of 4
     int radix_step;      // lines above 1024: kRadixDft or kRadixSums
 };
@@ -32,7 +32,7 @@ constexpr int kRadixSums = 2;
 // One batch of plane pairs resident on the device.  Pair p packs planes
 // 2p (real part) and 2p+1 (imaginary part).
 struct RlBatch {
-    float2 *C;            // npairs x H x W complex work planes, tiled 2 x 8
+    float2 *C;            // npairs x H x W complex work planes, row-major (see RowSwizzle)
     float2 *est;          // npairs x H x W (estimate of plane 2p, of plane 2p+1)
     const void *data;     // view v, plane z at data + (v * view_stride + z * plane_stride) samples
     size_t view_stride;

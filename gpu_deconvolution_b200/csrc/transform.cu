@@ -160,9 +160,6 @@ struct Source {
     int bx, by, bz;  // brick
 };
 
-// Status word of launches whose caller has none.
-__device__ int g_status;
-
 struct Brick {
     int ox, oy, oz;  // texel of the brick's first element
     int mode;        // 0: no brick (every texel from global memory); 1: brick, each load
@@ -236,8 +233,8 @@ __device__ __forceinline__ Brick load_brick(const CUtensorMap &tmap, const Sourc
                 __nanosleep(64);
         }
         b.mode = done ? (all_inside ? 2 : 1) : 0;
-        if (!done)
-            atomicExch(status ? status : &g_status, 1);
+        if (!done && status)  // the voxels come from global memory then
+            atomicExch(status, 1);
     }
     return b;
 }

@@ -498,8 +498,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
 // for the bias gradient; at the end all four read tensor memory and add the
 // sums with atomics, consecutive lanes consecutive ci.
 // The tensor cores' FP32 accumulation rounds towards zero: a sum of n pixels
-// comes out about 1.2e-9 n too small (3.7e-5 over 31.9 k pixels), so the share
-// of a CTA is bounded (launch_wgrad), and the bias
+// comes out about 1.2e-9 n too small.  A CTA's share (launch_wgrad) grows with
+// the batch: 31.9 k pixels, 3.7e-5, at 16 planes of 512 x 512, four times that
+// at 64.  The bias
 // sums, which cancel more, are ordinary FP32 additions (as an MMA with a
 // matrix of ones they were 4.7e-5 off).
 // Four 512 x 512 planes: 32 -> 32 channels 69 us (280 us with one tap per CTA),
@@ -830,7 +831,8 @@ bool launch_wgrad(const CUtensorMap &tx, const CUtensorMap &tg, const GemmArgs &
     if (!configure(k, C::SMEM, devices, sms))
         return false;
     const int ntiles = g.N * ((g.H + kGradH - 1) / kGradH) * ((g.W + kGradW - 1) / kGradW);
-    // pixels per CTA: a bounded accumulation (see the kernel), at least 8 tiles
+    // pixels per CTA: at least 8 tiles, and for larger batches so many that the
+    // grid covers the GPU a few times over
     const long long parts = (long long)g.taps * ((g.cout + 127) / 128) * ((g.cin + 255) / 256);
     const int chunk = (int)std::min<long long>(ntiles, std::max<long long>(8, (ntiles * parts + 1183) / 1184));
     const dim3 grid((ntiles + chunk - 1) / chunk, g.cout / BN, g.cin / (CB * GROUPS));

@@ -6,8 +6,8 @@
 //   1. an E-point DFT in registers over m              -> Y[t][k1]
 //   2. twiddle Y[t][k1] *= w_N^(t k1)                  (table, coalesced)
 //   3. transpose through shared memory: lane t takes the sequences
-//      k1 = t + T s (s < E/T); positions are XOR-swizzled so that both the
-//      write and the read of the transpose are free of bank conflicts
+//      k1 = t + T s (s < E/T); padded rows (row passes) or an XOR swizzle
+//      (the column tile) keep its write and its read free of bank conflicts
 //   4. a T-point DFT in registers over t for each of those sequences
 // giving X[k1 + E k2], which lands in lane t as v[m] = X[t + T m] again: the
 // same pattern as the input, so element-wise work between a transform and the
@@ -123,14 +123,6 @@ struct WarpFft {
     static constexpr int T = warp_fft_lanes(N);
     static constexpr int E = N / T;
     static constexpr int S = E / T;
-    // Shared-memory floats per group (real and imaginary planes).  The group
-    // size T is added so that the G = 32 / T groups of a warp start T banks
-    // apart: with the XOR swizzle below, every transpose write and read of a
-    // whole warp then touches 32 distinct banks.
-    static constexpr int group_floats = 2 * N + T;
-
-    // Position of transpose element (k1, t) inside a group's buffer.
-    static __device__ __forceinline__ int tpos(int k1, int t) { return k1 * T + (t ^ (k1 & (T - 1))); }
 
     // Twiddle table layout (per length N, built on the host, float2):
     //   [j * T + t]       = w_N^(R8 j t)   for j < J   (R8 = min(E, kWarpTwiddleRun), J = E / R8)
@@ -141,23 +133,6 @@ struct WarpFft {
     static constexpr int R8 = E < kWarpTwiddleRun ? E : kWarpTwiddleRun;
     static constexpr int J = E / R8;
     static constexpr int table_size = (J + 1) * T;
-
-    // In-place transform of v (lane pattern v[m] = x[t + T m]).
-    // tw: twiddle table above.  The transpose buffer element p lives at
-    // bre[p * STRIDE] / bim[p * STRIDE] (this group's shared memory); t: lane
-    // index inside the group.
-    // Transpose buffer element p at bre[p * STRIDE] / bim[p * STRIDE].
-    template <int STRIDE>
-    struct StridedAddr {
-        __device__ __forceinline__ int operator()(int p) const { return p * STRIDE; }
-    };
-
-    template <int DIR, int STRIDE = 1>
-    static __device__ __forceinline__ void run(float2 *v, const float2 *__restrict__ tw, float *bre, float *bim,
-                                               int t)
-    {
-        run_addr<DIR>(v, tw, bre, bim, t, StridedAddr<STRIDE>());
-    }
 
     // Step 2: v[k1] *= w_N^(t k1), k1 < E (table entries times a recurrence).
     template <int DIR>
@@ -212,7 +187,9 @@ struct WarpFft {
         __device__ __forceinline__ void operator()() const {}
     };
 
-    // The transform with the transpose through the padded float2 buffer buf.
+    // In-place transform of v (lane pattern v[m] = x[t + T m]), the transpose
+    // through the padded float2 buffer buf; tw: twiddle table above, t: lane
+    // index inside the group.
     // after_read() runs once every lane has read its transpose elements back,
     // when buf is free for other use until the next transform.
     template <int DIR, typename AfterRead = Nothing>
@@ -234,61 +211,6 @@ struct WarpFft {
                 v[s * T + j] = rd[s * T * (T + 1) + j];
         __syncwarp();
         after_read();
-#pragma unroll
-        for (int s = 0; s < S; s++)
-            Dft<T, DIR>::run(v + s * T);
-        reorder(v);
-    }
-
-    // Same, with the transpose element p at buf[addr(p)] (float2).
-    template <int DIR, typename Addr>
-    static __device__ __forceinline__ void run_addr2(float2 *v, const float2 *__restrict__ tw, float2 *buf, int t,
-                                                     const Addr &addr)
-    {
-        Dft<E, DIR>::run(v);
-        twiddle<DIR>(v, tw, t);
-#pragma unroll
-        for (int k1 = 0; k1 < E; k1++)
-            buf[addr(tpos(k1, t))] = v[k1];
-        __syncwarp();
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-            const int k1 = t + T * s;
-#pragma unroll
-            for (int j = 0; j < T; j++)
-                v[s * T + j] = buf[addr(tpos(k1, j))];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int s = 0; s < S; s++)
-            Dft<T, DIR>::run(v + s * T);
-        reorder(v);
-    }
-
-    // Same, with the transpose buffer element p at bre[addr(p)] / bim[addr(p)].
-    template <int DIR, typename Addr>
-    static __device__ __forceinline__ void run_addr(float2 *v, const float2 *__restrict__ tw, float *bre, float *bim,
-                                                    int t, const Addr &addr)
-    {
-        Dft<E, DIR>::run(v);
-        twiddle<DIR>(v, tw, t);
-#pragma unroll
-        for (int k1 = 0; k1 < E; k1++) {
-            const int p = addr(tpos(k1, t));
-            bre[p] = v[k1].x;
-            bim[p] = v[k1].y;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-            const int k1 = t + T * s;
-#pragma unroll
-            for (int j = 0; j < T; j++) {
-                const int p = addr(tpos(k1, j));
-                v[s * T + j] = make_float2(bre[p], bim[p]);
-            }
-        }
-        __syncwarp();
 #pragma unroll
         for (int s = 0; s < S; s++)
             Dft<T, DIR>::run(v + s * T);

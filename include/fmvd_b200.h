@@ -23,6 +23,8 @@ typedef struct fmvd_b200_plan fmvd_b200_plan;
 fmvd_b200_plan *fmvd_b200_plan_create(int bits, int dataH, int dataW, const float *const *h_Weights,
                                       float **h_Kernel, int kernelH, int kernelW, fmvd_psf_type iteration_type,
                                       int nViews, int pairs_per_batch);
+/* pairs_per_batch: the most a batch holds; where the caller left it to the
+ * library, long runs take smaller, even batches. */
 int fmvd_b200_plan_query(const fmvd_b200_plan *plan, int *fftH, int *fftW, int *pairs_per_batch);
 /* fmvd_b200_plan_create with the column-pass width as well: col_warps = 2, 4
  * or 8 warps (columns) per block for padded planes up to 1024 rows, 0 for
@@ -43,7 +45,8 @@ fmvd_b200_plan *fmvd_b200_plan_create_scheduled(int bits, int dataH, int dataW, 
 /* The plan's radix schedule (1 or 2, as above). */
 int fmvd_b200_plan_radix_step(const fmvd_b200_plan *plan);
 /* Column-pass warps per block of the plan (0 for planes above 1024 rows,
- * whose column pass has a fixed two-column tile). */
+ * whose column pass has a fixed four-column tile).  Where the caller left
+ * them to the library, launches of few planes below 1024 rows take half. */
 int fmvd_b200_plan_col_warps(const fmvd_b200_plan *plan);
 /* View v, plane z at d_views + (v * view_stride + z * dataH * dataW) samples;
  * output plane z at d_out + z * dataH * dataW.  d_estimate (optional)
