@@ -23,9 +23,10 @@
 // box with a one-pixel border.
 //
 // Every mbarrier wait is bounded: on a timeout the CTA records an error in
-// *status and finishes without hanging.  A role that runs on a whole warp
-// leaves its loops with all lanes together (warp_wait, warp_sees): its MMAs,
-// commits and tensor-memory loads wait for every lane of the warp.
+// *status and finishes without hanging.  A role ends at the first of its own
+// waits that gives up (the others' waits then run out too), and one that runs on
+// a whole warp with all lanes together (warp_wait): its MMAs, commits and
+// tensor-memory loads wait for every lane of the warp.
 #include "fmvd_internal.h"
 #include "smem_opt_in.h"
 #include "tma_util.cuh"
@@ -59,8 +60,6 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity)
 {
     return __all_sync(0xffffffffu, umma::bar_wait(bar, parity));
 }
-// Whether any lane of a whole, converged warp sees the flag another role raises.
-__device__ __forceinline__ bool warp_sees(int flag) { return __any_sync(0xffffffffu, flag); }
 
 // Sixteen bf16 values as floats (vec: p on a 32-byte boundary).
 __device__ __forceinline__ void load16(const bf16 *p, int vec, float (&f)[16])
@@ -240,20 +239,19 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- MMA issue
         const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
         int gk = 0, it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
             const int ab = it & 1;
-            if (it >= 2 && !warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
-                fail_sh = 1;
+            ok = it < 2 || warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1);
+            if (!ok)
                 break;
-            }
             umma::tc_fence_after();
             const uint32_t acc = tmem + ab * C::ACC_COLS;
             for (int kb = 0; kb < nk; kb++, gk++) {
                 const int s = gk % C::STAGES, round = gk / C::STAGES;
-                if (!warp_wait(&full[s], round & 1)) {
-                    fail_sh = 1;
+                ok = warp_wait(&full[s], round & 1);
+                if (!ok)
                     break;
-                }
                 umma::tc_fence_after();
                 const uint32_t a0 = umma::smem_addr(smem) + s * C::STAGE;
                 const umma::Desc ad = umma::make_desc(a0, 16, 8 * C::R, C::R);
@@ -265,11 +263,13 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
             }
             umma::mma_commit(&acc_full[ab]);
         }
+        if (!ok)
+            fail_sh = 1;
     } else {
         // ---- epilogue: warp w owns accumulator rows 32w..32w+31
         const int row = warp * 32 + lane;
         int it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
             const int ab = it & 1;
             if (!warp_wait(&acc_full[ab], (it >> 1) & 1)) {
                 fail_sh = 1;
@@ -404,28 +404,21 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         // ---- MMA issue
         const uint32_t idesc = umma::make_idesc(128, BN, 0, 0);
         const umma::Desc bd = umma::make_desc(umma::smem_addr(wsm), 16, 8 * C::R, C::R);
-        if (!warp_wait(&wfull, 0))
-            fail_sh = 1;
+        bool ok = warp_wait(&wfull, 0);
         int gs = 0, it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++, gs += NB) {
+        for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++, gs += NB) {
             const int ab = it & 1;
-            if (it >= 2 && !warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
-                fail_sh = 1;
-                break;
-            }
+            ok = it < 2 || warp_wait(&acc_empty[ab], ((it >> 1) - 1) & 1);
             const uint32_t acc = tmem + ab * C::ACC_COLS;
             umma::Desc ad[NB];
-            bool ok = true;
 #pragma unroll
             for (int cb = 0; cb < NB; cb++) {
                 const int s = (gs + cb) % C::SLOTS, round = (gs + cb) / C::SLOTS;
                 ok = ok && warp_wait(&full[s], round & 1);
                 ad[cb] = umma::make_desc(umma::smem_addr(slots) + s * C::SLOT, 16, kBoxW * C::R, C::R);
             }
-            if (!ok) {
-                fail_sh = 1;
+            if (!ok)
                 break;
-            }
             umma::tc_fence_after();
 #pragma unroll
             for (int t = 0; t < 9; t++)
@@ -441,11 +434,13 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
                 umma::mma_commit(&empty[(gs + cb) % C::SLOTS]);
             umma::mma_commit(&acc_full[ab]);
         }
+        if (!ok)
+            fail_sh = 1;
     } else {
         // ---- epilogue: warp w owns accumulator rows 32w..32w+31
         const int row = warp * 32 + lane;
         int it = 0;
-        for (int tile = blockIdx.x; tile < ntiles && !warp_sees(fail_sh); tile += gridDim.x, it++) {
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
             const int ab = it & 1;
             if (!warp_wait(&acc_full[ab], (it >> 1) & 1)) {
                 fail_sh = 1;
