@@ -199,13 +199,15 @@ def peak_hbm():
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the four
 # passes of one view update of a 6-plane batch of 1024 x 1024 planes, per
 # padded voxel, from one ncu capture of this workload's small case:
-#   ncu --set full --cache-control none --clock-control none \
-#       -k regex:"row_pass_w|col_pass_w" -s 40 -c 4 \
-#       python bench.py --small --steps 1 --warmup 1 --no-e2e --no-cpu
-# (22.1 MB per view update; the batch's work planes stay in L2).
-DRAM_BYTES_PER_PADDED_VOXEL_VIEW_UPDATE = 3.52
+#   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum,sm__inst_executed.sum \
+#       --cache-control none --clock-control none -k regex:"row_pass_w|col_pass_w" -s 40 -c 8 \
+#       python bench.py --small --steps 1 --warmup 1 --no-e2e --no-cpu --no-warmstart
+# (39 MB per view update, mean of two: the batch's work planes stay in L2, each
+# column pass reads its spectrum, 8.2 MB, from DRAM.  Captures that replay a
+# launch dozens of times find the spectrum in L2 and show 22 MB.)
+DRAM_BYTES_PER_PADDED_VOXEL_VIEW_UPDATE = 6.2
 # Thread instructions of the same four passes per padded voxel (the same
-# batch shape's sm__inst_executed.sum x 32 / padded voxels: 36.92 M warp
+# capture's sm__inst_executed.sum x 32 / padded voxels: 36.93 M warp
 # instructions per view update of the 6-plane batch).  With one warp
 # instruction per SM sub-partition per cycle (148 SMs x 4 x 32 lanes x clock)
 # this gives the issue-bound ceiling of the passes.

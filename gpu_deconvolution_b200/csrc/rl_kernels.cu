@@ -957,7 +957,7 @@ __device__ __forceinline__ void col_fft_512(float2 *v, const TW &tw, uint32_t wb
 constexpr int kLineColumns = 4;
 // Resident blocks per SM, which cap the registers of a thread.  A launch of at
 // most one block per multiprocessor has nothing to share an SM with, and takes
-// the kernel compiled for one (R = 3 to 5: 204 to 255 registers instead of 102
+// the kernel compiled for one (R = 3 to 5: 165 to 189 registers instead of 96
 // to 128, so more loads in flight per thread; from R = 6 on they are the same).
 // Five iterations of two views (us, shared / one block, and two columns per
 // block as before): one pair of 1536 x 256 (64 blocks) 437 / 280, 435; three of
